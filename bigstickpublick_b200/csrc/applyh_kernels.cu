@@ -16,6 +16,7 @@
 // (hmat * phase, src/bapplyhlibOMP.f90:1093-1095, :1269-1272) and promoted
 // to the vector type; FP32 vectors accumulate in FP32, FP64 vectors in FP64.
 
+#include <algorithm>
 #include <type_traits>
 
 #include "applyh_tile.cuh"
@@ -95,11 +96,15 @@ static int launch_one(bsg_ctx *ctx, const T *vin, T *vout, int ld, int v0, int a
     // the base pointer is 16-byte aligned
     const bool full = (ld == NB) && ((reinterpret_cast<uintptr_t>(vin) & 15u) == 0);
     cudaError_t e;
+    // the attribute belongs to the function, not the context: set to the
+    // hardware limit once per context, so that contexts of different sizes do
+    // not undo one another's
     auto allow = [&](const void *fn) -> cudaError_t {
         size_t &cur = ctx->smem_allowed[fn];
         if (cur >= smem) return cudaSuccess;
-        const cudaError_t r = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (r == cudaSuccess) cur = smem;
+        const size_t most = std::max<size_t>(smem, 227 * 1024);
+        const cudaError_t r = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
+        if (r == cudaSuccess) cur = most;
         return r;
     };
     auto go = [&](auto k) -> cudaError_t {
