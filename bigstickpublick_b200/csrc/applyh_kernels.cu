@@ -168,6 +168,7 @@ static int launch_typed(bsg_ctx *ctx, const T *vin, T *vout, int nb, int accumul
 }
 
 int launch_applyh_cols(bsg_ctx *ctx, const void *vin, double *cols, int nb, int prec, cudaStream_t s) {
+    if (cols && group_takes(ctx, nb, prec)) return launch_rowgroup(ctx, vin, nullptr, nb, prec, 0, s, nullptr, cols);
     if (ctx->args.max_nbd > 5120)
         return set_err(ctx, BSG_ERR_UNSUPPORTED, "a neutron sector jump has more than 5120 distinct (b,d) pairs");
     if ((reinterpret_cast<uintptr_t>(vin) & 15u) != 0 || !cols)
@@ -196,6 +197,7 @@ int launch_applyh_cols(bsg_ctx *ctx, const void *vin, double *cols, int nb, int 
 
 int launch_applyh(bsg_ctx *ctx, const void *vin, void *vout, int nb, int prec, int accumulate,
                   cudaStream_t s, TileLookup lk) {
+    if (group_takes(ctx, nb, prec)) return launch_rowgroup(ctx, vin, vout, nb, prec, accumulate, s, lk, nullptr);
     // the 8 per-warp PN tables must fit in shared memory beside the partial
     // sums (227 KB per CTA; 32 KB of partial sums at nb = 16, FP64)
     if (ctx->args.max_nbd > 5120)

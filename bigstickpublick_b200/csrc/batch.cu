@@ -32,13 +32,16 @@
 #include <type_traits>
 #include <vector>
 
-#include "applyh_tile.cuh"
+#include "rowgroup.cuh"
 #include "lanczos_kernels.h"
+#include "rowgroup.h"
 
 namespace bsg {
 
 struct BatchSys {
     RowArgs a;
+    GroupArgs g;        // grouped contexts, with their shared-memory layout
+    int32_t parts[2], accel[2], bufel[2];
     const void *vin;
     void *vout;
 };
@@ -109,6 +112,23 @@ __global__ void __launch_bounds__(kWarps * 32, ITEMS >= 4 ? 8 : 6) k_rows_batch_
                                                                    const BatchItem *__restrict__ items, int nitems,
                                                                    int *__restrict__ counter, int mstride) {
     rows_batch_body<float, ITEMS, (ITEMS >= 2)>(sys, items, nitems, counter, mstride);
+}
+
+// grouped contexts: one CTA per (system, row), heaviest first; the system's
+// descriptor is staged in shared memory
+template <typename T>
+__global__ void __launch_bounds__(256, 4) k_rowgroup_batch(const BatchSys *__restrict__ sys,
+                                                            const BatchItem *__restrict__ items) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ BatchSys S;
+    const BatchItem w = items[blockIdx.x];
+    for (int k = threadIdx.x; k < (int)(sizeof(BatchSys) / 4); k += blockDim.x)
+        reinterpret_cast<int *>(&S)[k] = reinterpret_cast<const int *>(sys + w.sys)[k];
+    __syncthreads();
+    const Tile t = S.a.tiles[w.tile];
+    constexpr int P = sizeof(T) == 8 ? 1 : 0;
+    row_group<T, 1, kStore>(S.a, S.g, S.parts[P], t.row, t.npos, (const T *)S.vin, 1, (T *)S.vout, nullptr,
+                            reinterpret_cast<T *>(smem), S.accel[P], S.bufel[P]);
 }
 
 template <typename T, int ITEMS>
@@ -353,10 +373,12 @@ struct bsg_batch {
     int items = 4;            // ITEMS of the batched row kernel (tile width 32*items)
     int ctas_per_sm = 4;
     int mstride = 4;
-    DevBuf sys, work, counter;
+    DevBuf sys, work, counter, workg;
     int nitems = 0;
+    int nitemsg = 0;          // (system, row) items of the grouped contexts
     int nsm = 148;
     bool tuned = false;
+    std::vector<BatchSys> hsys;   // host copy of the descriptors
 };
 
 namespace {
@@ -377,55 +399,87 @@ int berr(bsg_batch *b, int code, const std::string &m) {
 }
 
 int build_items(bsg_batch *b, int items) {
-    std::vector<BatchItem> all;
-    std::vector<int64_t> wt;
+    std::vector<BatchItem> all, allg;
+    std::vector<int64_t> wt, wtg;
     std::vector<BatchSys> sys(b->n);
     for (int s = 0; s < b->n; ++s) {
         bsg_ctx *c = b->ctx[s];
-        const TileSet *ts = get_tiles(c, 32 * items);
+        const int tp = c->grouped ? kRowTile : 32 * items;
+        const TileSet *ts = get_tiles(c, tp);
         if (!ts) return berr(b, BSG_ERR_NOMEM, "tile build failed: " + c->last_error);
         sys[s].a = c->args;
         sys[s].a.tiles = (const Tile *)ts->buf.p;
         sys[s].a.ntiles = ts->ntiles;
         sys[s].a.accumulate = 0;
+        sys[s].g = c->group;
+        for (int p = 0; p < 2 && c->grouped; ++p) {
+            const GroupShape x = group_shape(c, p ? 8 : 4, 1);
+            sys[s].parts[p] = x.parts;
+            sys[s].accel[p] = x.accel;
+            sys[s].bufel[p] = x.bufel;
+        }
         std::vector<Tile> tl;
-        build_tile_list(c, 32 * items, tl);
+        build_tile_list(c, tp, tl);
         for (size_t t = 0; t < tl.size(); ++t) {
-            all.push_back(BatchItem{s, (int32_t)t});
-            wt.push_back((int64_t)c->h_work[tl[t].row] * tl[t].npos / std::max(1, c->h_rowlen[tl[t].row]) + 1);
+            (c->grouped ? allg : all).push_back(BatchItem{s, (int32_t)t});
+            (c->grouped ? wtg : wt).push_back((int64_t)c->h_work[tl[t].row] * tl[t].npos / std::max(1, c->h_rowlen[tl[t].row]) + 1);
         }
     }
-    std::vector<size_t> ord(all.size());
-    std::iota(ord.begin(), ord.end(), 0);
-    std::stable_sort(ord.begin(), ord.end(), [&](size_t x, size_t y) { return wt[x] > wt[y]; });
-    std::vector<BatchItem> sorted(all.size());
-    for (size_t i = 0; i < ord.size(); ++i) sorted[i] = all[ord[i]];
+    auto heaviest = [](const std::vector<BatchItem> &v, const std::vector<int64_t> &w) {
+        std::vector<size_t> ord(v.size());
+        std::iota(ord.begin(), ord.end(), 0);
+        std::stable_sort(ord.begin(), ord.end(), [&](size_t x, size_t y) { return w[x] > w[y]; });
+        std::vector<BatchItem> sorted(v.size());
+        for (size_t i = 0; i < ord.size(); ++i) sorted[i] = v[ord[i]];
+        return sorted;
+    };
+    const std::vector<BatchItem> sorted = heaviest(all, wt), sortedg = heaviest(allg, wtg);
     int st;
     bsg_ctx *c0 = b->ctx[0];
     if ((st = upload(c0, b->sys, sys.data(), sizeof(BatchSys) * sys.size())) ||
-        (st = upload(c0, b->work, sorted.data(), sizeof(BatchItem) * sorted.size())))
+        (st = upload(c0, b->work, sorted.data(), sizeof(BatchItem) * sorted.size())) ||
+        (st = upload(c0, b->workg, sortedg.data(), sizeof(BatchItem) * sortedg.size())))
         return berr(b, st, c0->last_error);
     b->nitems = (int)sorted.size();
+    b->nitemsg = (int)sortedg.size();
+    b->hsys = std::move(sys);
     b->items = items;
     return BSG_OK;
 }
 
-// point every system's vin/vout at base + off (elements of size esize)
-int set_vectors(bsg_batch *b, const void *const *vin, void *const *vout) {
-    std::vector<BatchSys> sys(b->n);
-    if (cudaMemcpy(sys.data(), b->sys.p, sizeof(BatchSys) * b->n, cudaMemcpyDeviceToHost) != cudaSuccess)
-        return berr(b, BSG_ERR_CUDA, "batch descriptor download failed");
-    for (int s = 0; s < b->n; ++s) {
-        sys[s].vin = vin[s];
-        sys[s].vout = vout[s];
+// point every system's vin/vout at the given vectors, on the stream of the
+// launches that read them
+int set_vectors(bsg_batch *b, const void *const *vin, void *const *vout, cudaStream_t s) {
+    for (int k = 0; k < b->n; ++k) {
+        b->hsys[k].vin = vin[k];
+        b->hsys[k].vout = vout[k];
     }
-    if (cudaMemcpy(b->sys.p, sys.data(), sizeof(BatchSys) * b->n, cudaMemcpyHostToDevice) != cudaSuccess)
+    if (cudaMemcpyAsync(b->sys.p, b->hsys.data(), sizeof(BatchSys) * b->n, cudaMemcpyHostToDevice, s) != cudaSuccess)
         return berr(b, BSG_ERR_CUDA, "batch descriptor upload failed");
+    return BSG_OK;
+}
+
+template <typename T>
+int launch_batch_group(bsg_batch *b, cudaStream_t s) {
+    if (b->nitemsg == 0) return BSG_OK;
+    size_t smem = 0;
+    for (bsg_ctx *c : b->ctx)
+        if (c->grouped) smem = std::max(smem, group_shape(c, sizeof(T), 1).bytes(sizeof(T)));
+    auto kern = k_rowgroup_batch<T>;
+    cudaError_t e = smem > kGroupSmemMax ? cudaErrorInvalidValue
+                                         : cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGroupSmemMax);
+    if (e == cudaSuccess) {
+        kern<<<(unsigned)b->nitemsg, 256, smem, s>>>((const BatchSys *)b->sys.p, (const BatchItem *)b->workg.p);
+        e = cudaGetLastError();
+    }
+    if (e != cudaSuccess) return berr(b, BSG_ERR_CUDA, std::string("batched applyH: ") + cudaGetErrorString(e));
     return BSG_OK;
 }
 
 template <typename T, int ITEMS>
 int launch_batch_t(bsg_batch *b, cudaStream_t s) {
+    if (const int st = launch_batch_group<T>(b, s)) return st;
+    if (b->nitems == 0) return BSG_OK;
     const size_t smem = align16(sizeof(float) * (size_t)kWarps * b->mstride) + sizeof(T) * (size_t)kWarps * 32 * ITEMS;
     auto kern = batch_rows_kernel<T, ITEMS>();
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -526,6 +580,7 @@ int bsg_batch_destroy(bsg_batch *b) {
     if (b->stream) cudaStreamSynchronize(b->stream);
     dev_free(b->sys);
     dev_free(b->work);
+    dev_free(b->workg);
     dev_free(b->counter);
     for (bsg_ctx *c : b->ctx) bsg_destroy(c);
     if (b->stream) cudaStreamDestroy(b->stream);
@@ -565,7 +620,7 @@ int bsg_batch_system(const bsg_batch *b, int s, bsg_ctx **ctx) {
 int bsg_batch_applyh(bsg_batch *b, const void *const *vin, void *const *vout, int prec, void *stream) {
     if (!b || !vin || !vout || (prec != BSG_PREC_FP32 && prec != BSG_PREC_FP64)) return BSG_ERR_ARG;
     cudaSetDevice(b->device);
-    int st = set_vectors(b, vin, vout);
+    int st = set_vectors(b, vin, vout, (cudaStream_t)stream);
     if (st) return st;
     // stream: the caller's cudaStream_t; NULL is the legacy default stream
     return launch_batch(b, prec, (cudaStream_t)stream);
@@ -601,7 +656,7 @@ int bsg_batch_autotune(bsg_batch *b, int *items_out, int *ctas_out, double *best
     const int cand_ctas[] = {4, 8};
     for (int it : cand_items) {
         if ((st = build_items(b, it))) break;
-        if ((st = set_vectors(b, vi.data(), vo.data()))) break;
+        if ((st = set_vectors(b, vi.data(), vo.data(), b->stream))) break;
         for (int cps : cand_ctas) {
             b->ctas_per_sm = cps;
             launch_batch(b, BSG_PREC_FP32, b->stream);
@@ -736,7 +791,7 @@ int bsg_batch_lanczos(bsg_batch *b, const bsg_lanczos_params *p, double *evals, 
             vi[s] = (const char *)X.p + (size_t)esz * b->off[s];
             vo[s] = (char *)Y.p + (size_t)esz * b->off[s];
         }
-        st = set_vectors(b, vi.data(), vo.data());
+        st = set_vectors(b, vi.data(), vo.data(), b->stream);
     }
     if (!st && cudaMemsetAsync(itd.p, 0, sizeof(int), s0) != cudaSuccess) st = BSG_ERR_CUDA;
     if (!st && cudaMemsetAsync(fl.p, 0, 16 * (size_t)n, s0) != cudaSuccess) st = BSG_ERR_CUDA;

@@ -22,6 +22,8 @@
 #include <unordered_map>
 
 #include "bsg_internal.h"
+#include "host_parallel.h"
+#include "rowgroup.h"
 
 namespace bsg {
 
@@ -103,40 +105,6 @@ using namespace bsg;
 
 namespace {
 
-// fn(i) for every i in [0, n), on up to 32 host threads taking chunks of
-// `chunk` indices from a shared counter.  Callers write only to locations
-// that index i owns, so the result does not depend on the schedule.
-// max_threads 1 runs inline: small systems (and the many systems of a batch,
-// which are already set up on parallel host threads) skip the thread start-up.
-template <typename F>
-void parallel_for(int64_t n, int64_t chunk, F fn, int max_threads = 32) {
-    const int64_t nchunks = (n + chunk - 1) / chunk;
-    const unsigned hw = std::max(1u, std::min((unsigned)std::max(1, max_threads), std::thread::hardware_concurrency()));
-    const int nt = (int)std::min<int64_t>((int64_t)hw, nchunks);
-    if (nt <= 1) {
-        for (int64_t i = 0; i < n; ++i) fn(i);
-        return;
-    }
-    std::atomic<int64_t> next{0};
-    std::atomic<bool> oom{false};
-    auto work = [&]() {
-        try {
-            for (;;) {
-                const int64_t c = next.fetch_add(1);
-                if (c >= nchunks || oom) return;
-                const int64_t i1 = std::min(n, (c + 1) * chunk);
-                for (int64_t i = c * chunk; i < i1; ++i) fn(i);
-            }
-        } catch (const std::bad_alloc &) {
-            oom = true;   // reported to the caller below as an allocation failure
-        }
-    };
-    std::vector<std::thread> th;
-    for (int k = 1; k < nt; ++k) th.emplace_back(work);
-    work();
-    for (auto &x : th) x.join();
-    if (oom) throw std::bad_alloc();
-}
 // f() on its own host thread; join() waits and reports an allocation failure
 struct Task {
     std::thread th;
@@ -185,7 +153,7 @@ int derive(bsg_ctx *ctx, const bsg_tables *t, const bsg_tables3 *t3, bool do_upl
     const bool three = (t3 != nullptr);
     ctx->threebody = three;
     // host threads for the derivation only where it is worth their start-up
-    const int nthr = t->dimbasis >= (int64_t)1 << 20 ? 32 : 1;
+    const int nthr = t->dimbasis >= (int64_t)1 << 18 ? 32 : 1;
     // ---- basic presence and sizes
     if (t->dimbasis <= 0 || t->nsd_p <= 0 || t->nsd_n <= 0)
         return set_err(ctx, BSG_ERR_BAD_TABLE, "empty basis");
@@ -524,6 +492,8 @@ int derive(bsg_ctx *ctx, const bsg_tables *t, const bsg_tables3 *t3, bool do_upl
     int64_t ops3[4] = {0, 0, 0, 0};   // PPP, NNN, PPN, PNN
     struct PPBundle { int64_t ib, px0, px1, nx0, nx1; bool bwd; };
     std::vector<PPBundle> pp_bundles;
+    struct PNBundle { int64_t ib, px0, px1; int32_t id; bool bwd; };
+    std::vector<PNBundle> pn_bundles;
     // one proton-side PN-form contribution (PN, PPN, PNN) of the jump s1 -> s2
     auto pn_contrib = [&](int64_t s1, int32_t ri, int32_t rf, int32_t id, int32_t aoff, int32_t coff, int ph,
                           const std::string &what) -> int {
@@ -550,7 +520,7 @@ int derive(bsg_ctx *ctx, const bsg_tables *t, const bsg_tables3 *t3, bool do_upl
         for (int64_t ib = 0; ib < t->nbundles; ++ib) {
             const int op = t->optype[ib];
             const int64_t n = std::max<int64_t>(0, t->pxend[ib] - t->pxstart[ib] + 1);
-            if (op == BSG_OP_PN || op == BSG_OP_PPN || op == BSG_OP_PNN) npn += n;
+            if (op == BSG_OP_PPN || op == BSG_OP_PNN) npn += n;
             else if (op == BSG_OP_NN || op == BSG_OP_NNN) nnn += n;
             else if (op == BSG_OP_SPE) nspe += n;
         }
@@ -762,25 +732,8 @@ int derive(bsg_ctx *ctx, const bsg_tables *t, const bsg_tables3 *t3, bool do_upl
                             return set_err(ctx, BSG_ERR_OOB_INDEX, "cpnpair+dpnpair outside hmatpn" + where);
                     }
             }
-            for (int64_t x = px0; x <= px1; ++x) {
-                const int64_t s1 = bwd ? t->p1b_fsd[x - 1] : t->p1b_isd[x - 1];
-                const int32_t ri = bwd ? p1b_rf[x - 1] : p1b_ri[x - 1], rf = bwd ? p1b_ri[x - 1] : p1b_rf[x - 1];
-                if (ri < 0 || rf < 0)
-                    return set_err(ctx, BSG_ERR_OOB_INDEX, "p1b isd/fsd is not a pstart value" + where);
-                if (nops[id].nout > ctx->h_rowlen[rf] || nop_maxin[id] >= ctx->h_rowlen[ri])
-                    return set_err(ctx, BSG_ERR_OOB_INDEX, "PN neutron jump outside the row" + where);
-                const int ph = t->p1b_phase[x - 1];
-                if (ph != 1 && ph != -1) return set_err(ctx, BSG_ERR_BAD_TABLE, "p1b_phase not +-1" + where);
-                for (int32_t sb = 0; sb < nop_nsub[id]; ++sb) {
-                    PNContrib c{};
-                    c.q_off = s1;
-                    c.nop = id + sb;
-                    c.aoff = (int32_t)(t->p1b_cop[x - 1] + nl_p) * ld;
-                    c.coff = (int32_t)(t->p1b_dop[x - 1] + nl_p) * ld;
-                    c.php = (float)ph;
-                    pn.push_back({rf, c});
-                }
-            }
+            // the jumps become contributions after the loop, as for PP
+            pn_bundles.push_back({ib, px0, px1, id, bwd});
             ops[3] += (px1 - px0 + 1) * (nx1 - nx0 + 1);
         } else if (op == BSG_OP_SPE) {
             if (!t->call_spe || !t->pspe_h || !t->nspe_h)
@@ -847,6 +800,46 @@ int derive(bsg_ctx *ctx, const bsg_tables *t, const bsg_tables3 *t3, bool do_upl
         for (size_t j = 0; j < nb_pp; ++j)
             if (bst[j]) return set_err(ctx, bst[j], bmsg[j]);
     }
+    if (!pn_bundles.empty()) {
+        // PN bundles (src/bapplyhlibOMP.f90:1242-1442), one per task: a
+        // contribution per jump and sub-operator, in bundle and jump order (a
+        // two-body context: nothing else goes to `pn`)
+        const size_t nb_pn = pn_bundles.size();
+        std::vector<size_t> at0(nb_pn + 1, pn.size());
+        for (size_t j = 0; j < nb_pn; ++j)
+            at0[j + 1] = at0[j] + (size_t)(pn_bundles[j].px1 - pn_bundles[j].px0 + 1) * (size_t)nop_nsub[pn_bundles[j].id];
+        pn.resize(at0[nb_pn]);
+        std::vector<int> bst(nb_pn, BSG_OK);
+        std::vector<std::string> bmsg(nb_pn);
+        parallel_for((int64_t)nb_pn, 1, [&](int64_t j) {
+            const PNBundle &B = pn_bundles[j];
+            auto fail = [&](int code, const char *m) {
+                bst[j] = code;
+                bmsg[j] = std::string(m) + " (opbundle " + std::to_string(B.ib + 1) + ")";
+            };
+            size_t at = at0[j];
+            for (int64_t x = B.px0; x <= B.px1; ++x) {
+                const int64_t s1 = B.bwd ? t->p1b_fsd[x - 1] : t->p1b_isd[x - 1];
+                const int32_t ri = B.bwd ? p1b_rf[x - 1] : p1b_ri[x - 1], rf = B.bwd ? p1b_ri[x - 1] : p1b_rf[x - 1];
+                if (ri < 0 || rf < 0) return fail(BSG_ERR_OOB_INDEX, "p1b isd/fsd is not a pstart value");
+                if (nops[B.id].nout > ctx->h_rowlen[rf] || nop_maxin[B.id] >= ctx->h_rowlen[ri])
+                    return fail(BSG_ERR_OOB_INDEX, "PN neutron jump outside the row");
+                const int ph = t->p1b_phase[x - 1];
+                if (ph != 1 && ph != -1) return fail(BSG_ERR_BAD_TABLE, "p1b_phase not +-1");
+                for (int32_t sb = 0; sb < nop_nsub[B.id]; ++sb) {
+                    PNContrib c{};
+                    c.q_off = s1;
+                    c.nop = B.id + sb;
+                    c.aoff = (int32_t)(t->p1b_cop[x - 1] + nl_p) * ld;
+                    c.coff = (int32_t)(t->p1b_dop[x - 1] + nl_p) * ld;
+                    c.php = (float)ph;
+                    pn[at++] = {rf, c};
+                }
+            }
+        }, nthr);
+        for (size_t j = 0; j < nb_pn; ++j)
+            if (bst[j]) return set_err(ctx, bst[j], bmsg[j]);
+    }
     ctx->stats.n_ops_spe = ops[0];
     ctx->stats.n_ops_pp = ops[1];
     ctx->stats.n_ops_nn = ops[2];
@@ -893,7 +886,7 @@ int derive(bsg_ctx *ctx, const bsg_tables *t, const bsg_tables3 *t3, bool do_upl
     // labels do not fit, the NN entries stay zero and FP64 keeps the 8-byte
     // records (ctx->rec32_nn)
     const int64_t nmatnn_all = t->nmatnn + (three ? t3->nmatnnn : 0);
-    const bool pack32 = ctx->max_rowlen <= 65536 && max_nbd_all <= 32768;
+    const bool pack32 = ctx->max_rowlen <= 65535 && max_nbd_all <= 32768;
     const bool nn32 = pack32 && nmatnn_all <= 32768;
     ctx->rec32_nn = nn32;
     std::vector<uint32_t> sell32_all;
@@ -921,10 +914,10 @@ int derive(bsg_ctx *ctx, const bsg_tables *t, const bsg_tables3 *t3, bool do_upl
             nops[o].sell_base = nrec_tot;
             nops[o].slice_base = nslice_tot;
             nrec_tot += op_recs[o];
-            nslice_tot += (nops[o].nout + 31) / 32;
+            nslice_tot += (nops[o].nout + 31) / 32 + 1;   // and where the last slice ends
         }
-        sell_all.assign((size_t)nrec_tot, make_int2(0, 0));   // padding rows hold {0, 0}
-        if (pack32) sell32_all.assign((size_t)nrec_tot, 0u);
+        sell_all.resize((size_t)nrec_tot);
+        if (pack32) sell32_all.resize((size_t)nrec_tot);
         slice_off_all.assign((size_t)nslice_tot, 0);
         parallel_for(nop_all, 16, [&](int64_t o) {
             const NOp &op = nops[o];
@@ -936,6 +929,15 @@ int derive(bsg_ctx *ctx, const bsg_tables *t, const bsg_tables3 *t3, bool do_upl
                     width = std::max(width, ptr[32 * sl + l + 1] - ptr[32 * sl + l]);
                 slice_off_all[op.slice_base + sl] = (int32_t)off;
                 const size_t row0 = (size_t)(op.sell_base + off);
+                // unused places: the jump-group kernel reads them as a record
+                // of a position that it keeps zero (one past the operator's
+                // input positions, one past the longest row); the row-tile
+                // kernels count records and never read them
+                const int32_t zero_pos = op.kind == 1 ? nop_maxin[o] + 1 : ctx->max_rowlen;
+                for (size_t q = row0; q < row0 + (size_t)32 * width; ++q) {
+                    sell_all[q] = make_int2(zero_pos, 0);
+                    if (pack32) sell32_all[q] = (uint32_t)zero_pos;
+                }
                 for (int l = 0; l < 32 && 32 * sl + l < op.nout; ++l)
                     for (int32_t k = ptr[32 * sl + l]; k < ptr[32 * sl + l + 1]; ++k) {
                         int2 r;
@@ -957,6 +959,7 @@ int derive(bsg_ctx *ctx, const bsg_tables *t, const bsg_tables3 *t3, bool do_upl
                     }
                 off += (int64_t)32 * width;
             }
+            slice_off_all[op.slice_base + (op.nout + 31) / 32] = (int32_t)off;
         }, nthr);
     }
     const int W = kRowWarps;
@@ -993,7 +996,9 @@ int derive(bsg_ctx *ctx, const bsg_tables *t, const bsg_tables3 *t3, bool do_upl
                 const auto &c = spe[start[3][q]].second;
                 refs.push_back({(int64_t)(c.hi - c.lo + 1), 3, start[3][q]});
             }
-            std::stable_sort(refs.begin(), refs.end(), [](const Ref &x, const Ref &y) { return x.wgt > y.wgt; });
+            std::sort(refs.begin(), refs.end(), [](const Ref &x, const Ref &y) {
+                return x.wgt != y.wgt ? x.wgt > y.wgt : x.type != y.type ? x.type < y.type : x.idx < y.idx;
+            });
             int64_t load[kRowWarps] = {0};
             for (const Ref &f : refs) {
                 int best = 0;
@@ -1009,24 +1014,24 @@ int derive(bsg_ctx *ctx, const bsg_tables *t, const bsg_tables3 *t3, bool do_upl
     auto by_slot = [&](auto &v, const std::vector<uint8_t> &wv, std::vector<int32_t> &ptr, auto &flat,
                        std::vector<int32_t> *perm) {
         const int64_t nslot = nrows * W;
-        std::vector<int64_t> key(v.size());
-        parallel_for((int64_t)v.size(), 1 << 16, [&](int64_t i) { key[i] = (int64_t)v[i].first * W + wv[i]; }, nthr);
+        std::vector<int32_t> key(v.size());   // slots fit 31 bits (checked below)
+        parallel_for((int64_t)v.size(), 1 << 16, [&](int64_t i) { key[i] = v[i].first * W + wv[i]; }, nthr);
         ptr.assign(nslot + 1, 0);
-        for (int64_t k : key) ptr[k + 1]++;
+        for (int32_t k : key) ptr[k + 1]++;
         for (int64_t r = 0; r < nslot; ++r) ptr[r + 1] += ptr[r];
-        std::vector<size_t> idx(v.size());
+        std::vector<int32_t> idx(v.size());
         {
             std::vector<int32_t> fill(ptr.begin(), ptr.end() - 1);
-            for (size_t i = 0; i < v.size(); ++i) idx[fill[key[i]]++] = i;
+            for (size_t i = 0; i < v.size(); ++i) idx[fill[key[i]]++] = (int32_t)i;
         }
         flat.resize(v.size());
         if (perm) perm->resize(v.size());
         parallel_for((int64_t)idx.size(), 1 << 16, [&](int64_t k) {
             flat[k] = v[idx[k]].second;
-            if (perm) (*perm)[k] = (int32_t)idx[k];
+            if (perm) (*perm)[k] = idx[k];
         }, nthr);
     };
-    if (pp.size() > (size_t)INT32_MAX || pn.size() > (size_t)INT32_MAX)
+    if (pp.size() > (size_t)INT32_MAX || pn.size() > (size_t)INT32_MAX || nrows * W >= INT32_MAX)
         return set_err(ctx, BSG_ERR_UNSUPPORTED, "more than 2^31 row contributions");
     std::vector<int32_t> spe_ptr, pp_perm;
     std::vector<SPEContrib> h_spe;
@@ -1195,11 +1200,13 @@ int derive(bsg_ctx *ctx, const bsg_tables *t, const bsg_tables3 *t3, bool do_upl
     a.nspe = (const float *)ctx->nspe.p;
     a.ld_cpn = ld;
     a.ncpn = (int32_t)cpn32.size();
-    return BSG_OK;
+    const GroupSource gs{nops, nop_maxin, nptr_all, spe_ptr, pn};
+    return group_eligible(ctx, gs, pack32) ? build_groups(ctx, gs, nthr) : BSG_OK;
 }
 
 void free_ctx(bsg_ctx *ctx) {
     for (auto &b : ctx->raw) dev_free(b);
+    free_groups(ctx);
     DevBuf *bufs[] = {&ctx->row_off, &ctx->pp_ptr, &ctx->nn_ptr, &ctx->pn_ptr, &ctx->spe_ptr, &ctx->pp, &ctx->nn,
                       &ctx->pn, &ctx->spe, &ctx->nops, &ctx->nptr, &ctx->pnrec, &ctx->nnrec, &ctx->bd, &ctx->sell,
                       &ctx->sell32, &ctx->slice_off, &ctx->hmatpn,

@@ -125,6 +125,28 @@ struct RowArgs {
     int64_t cols_ld;
 };
 
+// ---- jump groups (rowgroup.cuh): the PN-form jumps in (row, operator) order
+struct GroupJump {
+    int64_t q_off;      // input row offset
+    int64_t v;          // its matrix-element row in vtab: one value per label pair
+};
+// one work item of a row; y = kind << 16 | count
+//   PN: x first jump, count 4, 2 or 1 jumps, z operator, w its input positions
+//   PP: x first contribution, count up to 32
+//   NN: z operator, count-th of w shares of its records
+//   SPE: x contribution
+enum { kItemPN = 0, kItemPP = 1, kItemNN = 2, kItemSPE = 3 };
+struct GroupItem {
+    int32_t x, y, z, w;
+};
+struct GroupArgs {
+    const GroupJump *jumps;
+    const GroupItem *items;
+    const int32_t *item_ptr;      // [nrows * kRowWarps + 1]: the rows' slots
+    const float *vtab;
+    int32_t zero_pos;             // position that unused NN record places read: the longest row's end
+};
+
 struct DevBuf {
     void *p = nullptr;
     size_t bytes = 0;
@@ -168,6 +190,11 @@ struct bsg_ctx {
     bsg::DevBuf sell32;
     bsg::DevBuf hmatpn, cpn, dpn, nspe, hmatpp_d, hmatnn_d;
     bsg::RowArgs args{};
+    // jump groups (grouped: the context has them; group_takes: who takes them)
+    bool grouped = false;
+    bsg::DevBuf g_buf;
+    bsg::GroupArgs group{};
+    int64_t group_nbd = 0, group_nin = 0;   // most label pairs, input positions of an operator
     std::map<int, bsg::TileSet> tiles;   // tile size -> tiles
     // largest dynamic shared memory already allowed per kernel function (the
     // attribute is set once per size, not on every launch)
@@ -212,6 +239,11 @@ void build_tile_list(const bsg_ctx *ctx, int tp, std::vector<Tile> &tiles);
 typedef const TileSet *(*TileLookup)(bsg_ctx *ctx, int tp);
 int launch_applyh(bsg_ctx *ctx, const void *vin, void *vout, int nb, int prec, int accumulate,
                   cudaStream_t s, TileLookup lookup = nullptr);
+// whether applyH on a block of nb vectors takes the jump groups
+bool group_takes(const bsg_ctx *ctx, int nb, int prec);
+// applyH of a grouped context: same arguments, cols != nullptr for FP64 columns
+int launch_rowgroup(bsg_ctx *ctx, const void *vin, void *vout, int nb, int prec, int accumulate, cudaStream_t s,
+                    TileLookup lookup, double *cols);
 // H x for an interleaved input x (nb <= 16, dense and 16-byte aligned), the
 // result written as nb FP64 columns of length dim starting at cols
 int launch_applyh_cols(bsg_ctx *ctx, const void *vin, double *cols, int nb, int prec, cudaStream_t s);
