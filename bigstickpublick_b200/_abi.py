@@ -222,8 +222,12 @@ def gpu_lib():
         lib.bsg_lanczos.restype = C.c_int
         lib.bsg_grad.argtypes = [vp, f64p, C.c_int, f64p, f64p, f64p, f64p, f64p]
         lib.bsg_grad.restype = C.c_int
+        lib.bsg_grad_rows.argtypes = [vp, f64p, C.c_int, f64p, f64p, f64p, f64p, f64p]
+        lib.bsg_grad_rows.restype = C.c_int
         lib.bsg_density1b.argtypes = [vp, C.POINTER(BsgDensityTables), f64p, C.c_int, f64p, f64p]
         lib.bsg_density1b.restype = C.c_int
+        lib.bsg_density1b_rows.argtypes = [vp, C.POINTER(BsgDensityTables), f64p, C.c_int, f64p, f64p]
+        lib.bsg_density1b_rows.restype = C.c_int
         lib.bsg_apply1b.argtypes = [vp, C.POINTER(BsgDensityTables), f64p, f64p, f64p, f64p, C.c_int]
         lib.bsg_apply1b.restype = C.c_int
         lib.bsg_get_stats.argtypes = [vp, C.POINTER(BsgStats)]

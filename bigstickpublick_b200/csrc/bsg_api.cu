@@ -69,6 +69,40 @@ int upload(bsg_ctx *ctx, DevBuf &b, const void *src, size_t bytes) {
     return BSG_OK;
 }
 
+int pool_alloc(bsg_ctx *ctx, DevBuf &b, size_t bytes, cudaStream_t s) {
+    {
+        std::lock_guard<std::mutex> lock(ctx->pool_mu);
+        if (!ctx->pool) {
+            cudaMemPoolProps props{};
+            props.allocType = cudaMemAllocationTypePinned;
+            props.location.type = cudaMemLocationTypeDevice;
+            props.location.id = ctx->device;
+            int st = cuda_check(ctx, cudaMemPoolCreate(&ctx->pool, &props), "cudaMemPoolCreate");
+            if (st) {
+                ctx->pool = nullptr;
+                return st;
+            }
+            uint64_t keep = kPoolKeep;
+            cudaMemPoolSetAttribute(ctx->pool, cudaMemPoolAttrReleaseThreshold, &keep);
+        }
+    }
+    b.bytes = bytes ? bytes : 16;
+    const int st = cuda_check(ctx, cudaMallocFromPoolAsync(&b.p, b.bytes, ctx->pool, s), "cudaMallocFromPoolAsync");
+    if (st) b = DevBuf{};
+    return st;
+}
+
+int pool_upload(bsg_ctx *ctx, DevBuf &b, const void *src, size_t bytes, cudaStream_t s) {
+    const int st = pool_alloc(ctx, b, bytes, s);
+    if (st || !bytes) return st;
+    return cuda_check(ctx, cudaMemcpyAsync(b.p, src, bytes, cudaMemcpyHostToDevice, s), "upload");
+}
+
+void pool_free(DevBuf &b, cudaStream_t s) {
+    if (b.p) cudaFreeAsync(b.p, s);
+    b = DevBuf{};
+}
+
 void build_tile_list(const bsg_ctx *ctx, int tp, std::vector<Tile> &tiles) {
     // tiles of tp positions, heaviest rows first (longest-processing-time order)
     std::vector<int32_t> order(ctx->nrows);
@@ -1220,6 +1254,8 @@ void free_ctx(bsg_ctx *ctx) {
     ctx->chunk_tiles.clear();
     for (cudaEvent_t e : ctx->chunk_ev) cudaEventDestroy(e);
     ctx->chunk_ev.clear();
+    if (ctx->pool) cudaMemPoolDestroy(ctx->pool);
+    ctx->pool = nullptr;
     if (ctx->copy_stream) cudaStreamDestroy(ctx->copy_stream);
     ctx->copy_stream = nullptr;
     if (ctx->ev0) cudaEventDestroy(ctx->ev0);

@@ -5,6 +5,7 @@
 #include <stdint.h>
 
 #include <map>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -222,6 +223,11 @@ struct bsg_ctx {
     std::map<int, bsg::ChunkTiles> chunk_tiles;
     cudaStream_t copy_stream = nullptr;
     std::vector<cudaEvent_t> chunk_ev;
+    // stream-ordered scratch of the state calls (adjoint, densities): the
+    // context's own pool, which keeps up to kPoolKeep between calls and goes
+    // with the context
+    std::mutex pool_mu;
+    cudaMemPool_t pool = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
 };
 
@@ -231,6 +237,11 @@ int cuda_check(bsg_ctx *ctx, cudaError_t e, const char *what);
 int dev_alloc(bsg_ctx *ctx, DevBuf &b, size_t bytes);
 void dev_free(DevBuf &b);
 int upload(bsg_ctx *ctx, DevBuf &b, const void *src, size_t bytes);
+// stream-ordered scratch from the context's pool; freed on the same stream
+constexpr uint64_t kPoolKeep = (uint64_t)1 << 30;
+int pool_alloc(bsg_ctx *ctx, DevBuf &b, size_t bytes, cudaStream_t s);
+int pool_upload(bsg_ctx *ctx, DevBuf &b, const void *src, size_t bytes, cudaStream_t s);
+void pool_free(DevBuf &b, cudaStream_t s);
 const TileSet *get_tiles(bsg_ctx *ctx, int tp);
 // row tiles of width tp in longest-processing-time order (host list)
 void build_tile_list(const bsg_ctx *ctx, int tp, std::vector<Tile> &tiles);
@@ -248,9 +259,9 @@ int launch_rowgroup(bsg_ctx *ctx, const void *vin, void *vout, int nb, int prec,
 // result written as nb FP64 columns of length dim starting at cols
 int launch_applyh_cols(bsg_ctx *ctx, const void *vin, double *cols, int nb, int prec, cudaStream_t s);
 // adjoint gradients of nsys systems x nstates states in one launch
-// (grad.cu); evecs[s] host dim_s x nstates column-major; outputs host
+// (grad.cu); evecs[s] host dim_s x nstates, column-major or (rows) row-major; outputs host
 // [state][label] per system (dspe_* may be null); kernel_ms: device time
 int grad_many(bsg_ctx *const *ctxs, int nsys, const double *const *evecs, int nstates, double *const *dpp,
               double *const *dnn, double *const *dpn, double *const *dspe_p, double *const *dspe_n, cudaStream_t s,
-              std::string &err, double *kernel_ms);
+              std::string &err, double *kernel_ms, bool rows = false);
 }  // namespace bsg

@@ -60,6 +60,16 @@ __global__ void k_interleave(const double *__restrict__ cols, double *__restrict
     }
 }
 
+// the same from [dim x ns] row-major (odd ns; even rows need no padding)
+__global__ void k_pad_rows(const double *__restrict__ rows, double *__restrict__ x, int64_t dim, int ns, int nsp) {
+    const int64_t n = dim * nsp;
+    for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n; e += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t row = e / nsp;
+        const int k = (int)(e - row * nsp);
+        x[e] = k < ns ? rows[row * ns + k] : 0.0;
+    }
+}
+
 __host__ __device__ inline int den_nsp(int ns) { return (ns + 1) & ~1; }
 // rows staged per pass: tile * nsp <= 1024 doubles per side and buffer, so
 // that 32 KB of shared memory per CTA leaves room for 6 CTAs per SM
@@ -390,8 +400,10 @@ __global__ void __launch_bounds__(256) k_apply1b_t(const AGroup *__restrict__ gr
 
 using namespace bsg;
 
-extern "C" int bsg_density1b(bsg_ctx *ctx, const bsg_density_tables *dt, const double *vecs, int nstates,
-                             double *p1bopme, double *n1bopme) {
+// rows: vecs is dim x nstates row-major (the layout the kernel stages), else
+// column-major
+static int density1b(bsg_ctx *ctx, const bsg_density_tables *dt, const double *vecs, int nstates, double *p1bopme,
+                     double *n1bopme, bool rows) {
     if (!ctx) return BSG_ERR_ARG;
     if (!dt || !vecs || !p1bopme || !n1bopme)
         return set_err(ctx, BSG_ERR_ARG, "bsg_density1b: null argument");
@@ -456,29 +468,31 @@ extern "C" int bsg_density1b(bsg_ctx *ctx, const bsg_density_tables *dt, const d
 
     // ---- device work
     DevBuf d_cols, d_x, d_segs, d_chunks, d_part, d_l0, d_lid, d_outp, d_outn;
+    cudaStream_t s = ctx->stream;
     auto release = [&]() {
-        dev_free(d_cols); dev_free(d_x); dev_free(d_segs); dev_free(d_chunks); dev_free(d_part);
-        dev_free(d_l0); dev_free(d_lid); dev_free(d_outp); dev_free(d_outn);
+        for (DevBuf *b : {&d_cols, &d_x, &d_segs, &d_chunks, &d_part, &d_l0, &d_lid, &d_outp, &d_outn}) pool_free(*b, s);
     };
     const size_t vbytes = sizeof(double) * (size_t)dim * ns;
-    if ((st = dev_alloc(ctx, d_cols, vbytes)) || (st = dev_alloc(ctx, d_x, sizeof(double) * (size_t)dim * den_nsp(ns))) ||
-        (st = upload(ctx, d_segs, segs.data(), sizeof(DSeg) * segs.size())) ||
-        (st = upload(ctx, d_chunks, chunks.data(), sizeof(DChunk) * chunks.size())) ||
-        (st = dev_alloc(ctx, d_part, sizeof(double) * (size_t)np * chunks.size())) ||
-        (st = upload(ctx, d_l0, lab_chunk0.data(), sizeof(int32_t) * lab_chunk0.size())) ||
-        (st = upload(ctx, d_lid, lab_ids.data(), sizeof(int32_t) * lab_ids.size())) ||
-        (st = dev_alloc(ctx, d_outp, sizeof(double) * (size_t)np * std::max(1, nlab_p))) ||
-        (st = dev_alloc(ctx, d_outn, sizeof(double) * (size_t)np * std::max(1, nlab_n)))) {
+    const bool direct = rows && ns == den_nsp(ns);   // already as staged
+    if ((!direct && (st = pool_alloc(ctx, d_cols, vbytes, s))) ||
+        (st = pool_alloc(ctx, d_x, sizeof(double) * (size_t)dim * den_nsp(ns), s)) ||
+        (st = pool_upload(ctx, d_segs, segs.data(), sizeof(DSeg) * segs.size(), s)) ||
+        (st = pool_upload(ctx, d_chunks, chunks.data(), sizeof(DChunk) * chunks.size(), s)) ||
+        (st = pool_alloc(ctx, d_part, sizeof(double) * (size_t)np * chunks.size(), s)) ||
+        (st = pool_upload(ctx, d_l0, lab_chunk0.data(), sizeof(int32_t) * lab_chunk0.size(), s)) ||
+        (st = pool_upload(ctx, d_lid, lab_ids.data(), sizeof(int32_t) * lab_ids.size(), s)) ||
+        (st = pool_alloc(ctx, d_outp, sizeof(double) * (size_t)np * std::max(1, nlab_p), s)) ||
+        (st = pool_alloc(ctx, d_outn, sizeof(double) * (size_t)np * std::max(1, nlab_n), s))) {
         release();
         return st;
     }
-    cudaStream_t s = ctx->stream;
-    cudaError_t e = cudaMemcpyAsync(d_cols.p, vecs, vbytes, cudaMemcpyHostToDevice, s);
+    cudaError_t e = cudaMemcpyAsync(direct ? d_x.p : d_cols.p, vecs, vbytes, cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess) e = cudaMemsetAsync(d_outp.p, 0, d_outp.bytes, s);
     if (e == cudaSuccess) e = cudaMemsetAsync(d_outn.p, 0, d_outn.bytes, s);
     if (e == cudaSuccess) e = cudaEventRecord(ctx->ev0, s);
-    if (e == cudaSuccess) {
-        k_interleave<<<148 * 8, 256, 0, s>>>((const double *)d_cols.p, (double *)d_x.p, dim, ns, den_nsp(ns));
+    if (e == cudaSuccess && !direct) {
+        auto lay = rows ? k_pad_rows : k_interleave;
+        lay<<<148 * 8, 256, 0, s>>>((const double *)d_cols.p, (double *)d_x.p, dim, ns, den_nsp(ns));
         e = cudaGetLastError();
     }
     if (e == cudaSuccess) {
@@ -507,11 +521,21 @@ extern "C" int bsg_density1b(bsg_ctx *ctx, const bsg_density_tables *dt, const d
     if (e == cudaSuccess) {
         ctx->stats.density_ms = ms;
         ctx->stats.density_rows = total;
-        ctx->stats.density_launches = 3;
+        ctx->stats.density_launches = direct ? 2 : 3;
     }
     st = cuda_check(ctx, e, "bsg_density1b");
     release();
     return st;
+}
+
+extern "C" int bsg_density1b(bsg_ctx *ctx, const bsg_density_tables *dt, const double *vecs, int nstates,
+                             double *p1bopme, double *n1bopme) {
+    return density1b(ctx, dt, vecs, nstates, p1bopme, n1bopme, false);
+}
+
+extern "C" int bsg_density1b_rows(bsg_ctx *ctx, const bsg_density_tables *dt, const double *vecs, int nstates,
+                                  double *p1bopme, double *n1bopme) {
+    return density1b(ctx, dt, vecs, nstates, p1bopme, n1bopme, true);
 }
 
 extern "C" int bsg_apply1b(bsg_ctx *ctx, const bsg_density_tables *dt, const double *ppot, const double *npot,

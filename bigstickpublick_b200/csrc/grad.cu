@@ -31,6 +31,15 @@ __global__ void k_fix_to_double(const unsigned long long *__restrict__ acc, doub
         out[i] = fix_value(acc + 2 * i);
 }
 
+// [dim x ns] row-major -> column-major; a warp takes 32 states, whose lines
+// stay in L1 between the columns
+__global__ void k_rows_to_cols(const double *__restrict__ x, int64_t dim, int ns, double *__restrict__ y) {
+    const int lane = threadIdx.x & 31;
+    for (int64_t r = ((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5) * 32 + lane; r < dim;
+         r += (int64_t)gridDim.x * blockDim.x)
+        for (int k = 0; k < ns; ++k) y[(int64_t)k * dim + r] = __ldg(x + r * ns + k);
+}
+
 template <int ITEMS>
 __global__ void __launch_bounds__(kGradWarps * 32) k_grad_items(const GradDesc *__restrict__ desc,
                                                                 const GradItem *__restrict__ items, int mstride) {
@@ -48,7 +57,7 @@ constexpr int kGradItems = 4;  // 128-position tiles
 
 int grad_many(bsg_ctx *const *ctxs, int nsys, const double *const *evecs, int nstates, double *const *dpp,
               double *const *dnn, double *const *dpn, double *const *dspe_p, double *const *dspe_n, cudaStream_t s,
-              std::string &err, double *kernel_ms) {
+              std::string &err, double *kernel_ms, bool rows) {
     auto fail = [&](int code, const std::string &m) {
         err = m;
         return code;
@@ -89,14 +98,15 @@ int grad_many(bsg_ctx *const *ctxs, int nsys, const double *const *evecs, int ns
         for (int t = 0; t < ts[s2]->ntiles; ++t)
             for (int k = 0; k < nstates; ++k) items.push_back(GradItem{s2 * nstates + k, t});
     bsg_ctx *c0 = ctxs[0];
-    DevBuf psi, acc, out, descb, itemb;
+    DevBuf psi, tmp, acc, out, descb, itemb;
     auto cleanup = [&]() {
-        dev_free(psi); dev_free(acc); dev_free(out); dev_free(descb); dev_free(itemb);
+        for (DevBuf *b : {&psi, &tmp, &acc, &out, &descb, &itemb}) pool_free(*b, s);
     };
     int st;
-    if ((st = dev_alloc(c0, psi, sizeof(double) * (size_t)std::max<int64_t>(npsi, 1))) ||
-        (st = dev_alloc(c0, acc, 16 * (size_t)std::max<int64_t>(nacc, 1))) ||
-        (st = dev_alloc(c0, out, sizeof(double) * (size_t)std::max<int64_t>(nacc, 1)))) {
+    if (nstates == 1) rows = false;   // the same layout
+    if ((st = pool_alloc(c0, psi, sizeof(double) * (size_t)npsi, s)) ||
+        (rows && (st = pool_alloc(c0, tmp, sizeof(double) * (size_t)npsi, s))) ||
+        (st = pool_alloc(c0, acc, 16 * (size_t)nacc, s)) || (st = pool_alloc(c0, out, sizeof(double) * (size_t)nacc, s))) {
         cleanup();
         return fail(st, "device allocation: " + c0->last_error);
     }
@@ -122,15 +132,21 @@ int grad_many(bsg_ctx *const *ctxs, int nsys, const double *const *evecs, int ns
             d.psi = (const double *)psi.p + psi_off[s2] + (int64_t)k * c->dim;
         }
     }
-    if ((st = upload(c0, descb, desc.data(), sizeof(GradDesc) * desc.size())) ||
-        (st = upload(c0, itemb, items.data(), sizeof(GradItem) * std::max<size_t>(items.size(), 1)))) {
+    if ((st = pool_upload(c0, descb, desc.data(), sizeof(GradDesc) * desc.size(), s)) ||
+        (st = pool_upload(c0, itemb, items.data(), sizeof(GradItem) * items.size(), s))) {
         cleanup();
         return fail(st, "upload: " + c0->last_error);
     }
     cudaError_t e = cudaSuccess;
     for (int s2 = 0; s2 < nsys && e == cudaSuccess; ++s2)
-        e = cudaMemcpyAsync((double *)psi.p + psi_off[s2], evecs[s2], sizeof(double) * ctxs[s2]->dim * nstates,
-                            cudaMemcpyHostToDevice, s);
+        e = cudaMemcpyAsync((double *)(rows ? tmp.p : psi.p) + psi_off[s2], evecs[s2],
+                            sizeof(double) * ctxs[s2]->dim * nstates, cudaMemcpyHostToDevice, s);
+    for (int s2 = 0; rows && s2 < nsys && e == cudaSuccess; ++s2) {
+        const int64_t dim = ctxs[s2]->dim;
+        k_rows_to_cols<<<(unsigned)std::min<int64_t>((dim + 255) / 256, 148 * 8), 256, 0, s>>>(
+            (const double *)tmp.p + psi_off[s2], dim, nstates, (double *)psi.p + psi_off[s2]);
+        e = cudaGetLastError();
+    }
     if (e == cudaSuccess) e = cudaMemsetAsync(acc.p, 0, acc.bytes, s);
     const size_t smem = grad_smem_bytes(mstride);
     if (e == cudaSuccess)
@@ -150,27 +166,29 @@ int grad_many(bsg_ctx *const *ctxs, int nsys, const double *const *evecs, int ns
         e = cudaGetLastError();
     }
     cudaEventRecord(e1, s);
-    // outputs: per system, state-major blocks [state][label]
+    // one copy back, then per system state-major blocks [state][label]
+    std::vector<double> host((size_t)nacc);
+    if (e == cudaSuccess && nacc > 0)
+        e = cudaMemcpyAsync(host.data(), out.p, sizeof(double) * (size_t)nacc, cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     for (int s2 = 0; s2 < nsys && e == cudaSuccess; ++s2) {
         bsg_ctx *c = ctxs[s2];
         const bool spe = c->t.call_spe && dspe_p && dspe_n && dspe_p[s2] && dspe_n[s2];
-        for (int k = 0; k < nstates && e == cudaSuccess; ++k) {
-            const double *o = (const double *)out.p + acc_off[(size_t)s2 * nstates + k];
-            auto cp = [&](double *dst, const double *src, int64_t cnt) {
-                if (e == cudaSuccess && cnt > 0)
-                    e = cudaMemcpyAsync(dst, src, sizeof(double) * cnt, cudaMemcpyDeviceToHost, s);
+        for (int k = 0; k < nstates; ++k) {
+            const double *o = host.data() + acc_off[(size_t)s2 * nstates + k];
+            auto cp = [&](double *dst, int64_t cnt) {
+                std::copy(o, o + cnt, dst);
+                o += cnt;
             };
-            cp(dpp[s2] + k * c->t.nmatpp, o, c->t.nmatpp);
-            cp(dnn[s2] + k * c->t.nmatnn, o + c->t.nmatpp, c->t.nmatnn);
-            cp(dpn[s2] + k * c->t.nmatpn, o + c->t.nmatpp + c->t.nmatnn, c->t.nmatpn);
+            cp(dpp[s2] + k * c->t.nmatpp, c->t.nmatpp);
+            cp(dnn[s2] + k * c->t.nmatnn, c->t.nmatnn);
+            cp(dpn[s2] + k * c->t.nmatpn, c->t.nmatpn);
             if (spe) {
-                const int64_t b0 = c->t.nmatpp + c->t.nmatnn + c->t.nmatpn;
-                cp(dspe_p[s2] + k * c->t.nsd_p, o + b0, c->t.nsd_p);
-                cp(dspe_n[s2] + k * c->t.nsd_n, o + b0 + c->t.nsd_p, c->t.nsd_n);
+                cp(dspe_p[s2] + k * c->t.nsd_p, c->t.nsd_p);
+                cp(dspe_n[s2] + k * c->t.nsd_n, c->t.nsd_n);
             }
         }
     }
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (kernel_ms && e == cudaSuccess) {
         float ms = 0.f;
         cudaEventElapsedTime(&ms, e0, e1);
@@ -188,8 +206,8 @@ int grad_many(bsg_ctx *const *ctxs, int nsys, const double *const *evecs, int ns
 
 using namespace bsg;
 
-extern "C" int bsg_grad(bsg_ctx *ctx, const double *evecs, int nstates, double *dpp, double *dnn, double *dpn,
-                        double *dspe_p, double *dspe_n) {
+static int grad_one(bsg_ctx *ctx, const double *evecs, int nstates, double *dpp, double *dnn, double *dpn, double *dspe_p,
+                    double *dspe_n, bool rows) {
     if (!ctx) return BSG_ERR_ARG;
     if (!evecs || nstates < 1 || !dpp || !dnn || !dpn)
         return set_err(ctx, BSG_ERR_ARG, "bsg_grad: null argument or nstates < 1");
@@ -200,8 +218,18 @@ extern "C" int bsg_grad(bsg_ctx *ctx, const double *evecs, int nstates, double *
     double *p[1] = {dpp}, *nn[1] = {dnn}, *pn[1] = {dpn}, *sp[1] = {dspe_p}, *sn[1] = {dspe_n};
     std::string err;
     double ms = 0.0;
-    st = grad_many(cs, 1, ev, nstates, p, nn, pn, sp, sn, ctx->stream, err, &ms);
+    st = grad_many(cs, 1, ev, nstates, p, nn, pn, sp, sn, ctx->stream, err, &ms, rows);
     if (st) return set_err(ctx, st, "bsg_grad: " + err);
     ctx->stats.grad_ms = ms;
     return BSG_OK;
+}
+
+extern "C" int bsg_grad(bsg_ctx *ctx, const double *evecs, int nstates, double *dpp, double *dnn, double *dpn,
+                        double *dspe_p, double *dspe_n) {
+    return grad_one(ctx, evecs, nstates, dpp, dnn, dpn, dspe_p, dspe_n, false);
+}
+
+extern "C" int bsg_grad_rows(bsg_ctx *ctx, const double *evecs, int nstates, double *dpp, double *dnn, double *dpn,
+                             double *dspe_p, double *dspe_n) {
+    return grad_one(ctx, evecs, nstates, dpp, dnn, dpn, dspe_p, dspe_n, true);
 }

@@ -264,6 +264,10 @@ int  bsg_lanczos(bsg_ctx *ctx, const bsg_lanczos_params *p, const double *pivot_
  *      dspe_n[nstates*nsd_n] (the last two only when call_spe; may be NULL). ---- */
 int  bsg_grad(bsg_ctx *ctx, const double *evecs, int nstates,
               double *dpp, double *dnn, double *dpn, double *dspe_p, double *dspe_n);
+/* the same from eigenvectors stored dim x nstates row-major (all states of one
+ * basis state side by side) */
+int  bsg_grad_rows(bsg_ctx *ctx, const double *evecs, int nstates,
+              double *dpp, double *dnn, double *dpn, double *dspe_p, double *dspe_n);
 /*      All states in one launch; every label's sum is accumulated exactly (to
  *      2^-64) in 128-bit fixed point with integer atomics, so the result is
  *      bitwise repeatable and independent of how the work is split. */
@@ -308,6 +312,9 @@ typedef struct bsg_density_tables {
     const int64_t *pxstart, *pxend, *nxstart, *nxend, *cstride;
 } bsg_density_tables;
 int  bsg_density1b(bsg_ctx *ctx, const bsg_density_tables *dt, const double *vecs, int nstates,
+                   double *p1bopme, double *n1bopme);
+/* the same from vectors stored dim x nstates row-major */
+int  bsg_density1b_rows(bsg_ctx *ctx, const bsg_density_tables *dt, const double *vecs, int nstates,
                    double *p1bopme, double *n1bopme);
 
 /* ---- one-body operator: replaces master_apply1bop (src/bdenslib1.f90:2612)
