@@ -1376,16 +1376,24 @@ namespace {
 
 // host-pointer applyH in kChunks row-range chunks when the output is at least
 // kChunkBytes: each chunk's states are final when its launch ends, so their
-// copy back overlaps the launches after it
+// copy back overlaps the launches after it.  The row kernel, with kChunkRows
+// rows and more (a chunk's launch still fills the chip), is cut from
+// kGroupChunkBytes on.  Store / accumulate calls, whole -> chunked, pageable
+// memory: pf 4p4n FP32 (7.9 MB) 1.86 -> 1.67 / 2.65 -> 1.87 ms, FP64 3.16 -> 2.80
+// / 4.65 -> 3.26 ms, pf 4p4n 2Jz = 8 FP32 (5.6 MB) 1.35 -> 1.29 / 1.94 -> 1.44 ms.
 constexpr int kChunks = 4;
 constexpr size_t kChunkBytes = (size_t)32 << 20;
+constexpr size_t kGroupChunkBytes = (size_t)4 << 20;
+constexpr int kChunkRows = kChunks * 148 * 4;
 
-// the chunked tiles of width tp: rows cut into kChunks contiguous ranges of
-// about equal estimated work, each range's tiles heaviest row first
-const ChunkTiles *get_chunk_tiles(bsg_ctx *ctx, int tp) {
-    auto it = ctx->chunk_tiles.find(tp);
-    if (it != ctx->chunk_tiles.end()) return &it->second;
-    ChunkTiles ct;
+bool chunked(const bsg_ctx *ctx, size_t bytes, int nb, int prec) {
+    if (ctx->nrows < kChunks) return false;
+    if (bytes >= kChunkBytes) return true;
+    return bytes >= kGroupChunkBytes && ctx->nrows >= kChunkRows && group_takes(ctx, nb, prec);
+}
+
+// kChunks contiguous row ranges of about equal estimated work
+std::vector<int32_t> chunk_rows(const bsg_ctx *ctx) {
     int64_t total = 0;
     for (int32_t r = 0; r < ctx->nrows; ++r) total += ctx->h_work[r];
     std::vector<int32_t> rcut(1, 0);
@@ -1396,15 +1404,34 @@ const ChunkTiles *get_chunk_tiles(bsg_ctx *ctx, int tp) {
     }
     while ((int)rcut.size() <= kChunks) rcut.push_back(ctx->nrows);
     rcut.back() = ctx->nrows;
+    return rcut;
+}
+
+// the first state of each range, and the dimension
+std::vector<int64_t> chunk_states(const bsg_ctx *ctx) {
+    const std::vector<int32_t> rcut = chunk_rows(ctx);
+    std::vector<int64_t> cut(1, 0);
+    for (int c = 0; c < kChunks; ++c) {
+        int64_t n = cut.back();
+        for (int32_t r = rcut[c]; r < rcut[c + 1]; ++r) n += ctx->h_rowlen[r];
+        cut.push_back(n);
+    }
+    return cut;
+}
+
+// the chunked tiles of width tp, each range's tiles heaviest row first
+const ChunkTiles *get_chunk_tiles(bsg_ctx *ctx, int tp) {
+    auto it = ctx->chunk_tiles.find(tp);
+    if (it != ctx->chunk_tiles.end()) return &it->second;
+    ChunkTiles ct;
+    const std::vector<int32_t> rcut = chunk_rows(ctx);
     std::vector<Tile> tiles;
-    int64_t state = 0;
     for (int c = 0; c < kChunks; ++c) {
         std::vector<int32_t> order;
         for (int32_t r = rcut[c]; r < rcut[c + 1]; ++r) order.push_back(r);
         std::stable_sort(order.begin(), order.end(),
                          [&](int32_t x, int32_t y) { return ctx->h_work[x] > ctx->h_work[y]; });
         ct.start.push_back((int32_t)tiles.size());
-        ct.s0.push_back(state);
         for (int32_t r : order)
             for (int32_t p0 = 0; p0 < ctx->h_rowlen[r]; p0 += tp) {
                 Tile t;
@@ -1414,10 +1441,8 @@ const ChunkTiles *get_chunk_tiles(bsg_ctx *ctx, int tp) {
                 t.pad = 0;
                 tiles.push_back(t);
             }
-        for (int32_t r = rcut[c]; r < rcut[c + 1]; ++r) state += ctx->h_rowlen[r];
     }
     ct.start.push_back((int32_t)tiles.size());
-    ct.s0.push_back(state);
     if (upload(ctx, ct.buf, tiles.data(), tiles.size() * sizeof(Tile))) return nullptr;
     for (int c = 0; c < kChunks; ++c) {
         TileSet v;
@@ -1437,13 +1462,6 @@ const TileSet *chunk_lookup(bsg_ctx *ctx, int tp) {
     return ct ? &ct->view[t_chunk] : nullptr;
 }
 
-// states of chunk c for the launch's tile width: every tile width cuts the
-// rows the same way (the cut depends on the rows only), so any cached entry
-// gives the ranges
-const ChunkTiles *any_chunk_tiles(bsg_ctx *ctx) {
-    return ctx->chunk_tiles.empty() ? nullptr : &ctx->chunk_tiles.begin()->second;
-}
-
 int applyh_on(bsg_ctx *ctx, const void *vin, void *vout, int nb, int prec, int flags, cudaStream_t s) {
     if (!vin || !vout || nb < 1 || nb > 64 || (prec != BSG_PREC_FP32 && prec != BSG_PREC_FP64))
         return set_err(ctx, BSG_ERR_ARG, "bsg_applyh: bad arguments");
@@ -1457,10 +1475,12 @@ int applyh_on(bsg_ctx *ctx, const void *vin, void *vout, int nb, int prec, int f
     if (ctx->scratch_in.bytes < bytes) {
         if ((st = dev_alloc(ctx, ctx->scratch_in, bytes)) || (st = dev_alloc(ctx, ctx->scratch_out, bytes))) return st;
     }
+    const bool whole = !chunked(ctx, bytes, nb, prec);
     st = cuda_check(ctx, cudaMemcpyAsync(ctx->scratch_in.p, vin, bytes, cudaMemcpyHostToDevice, s), "H2D vin");
-    if (!st && acc) st = cuda_check(ctx, cudaMemcpyAsync(ctx->scratch_out.p, vout, bytes, cudaMemcpyHostToDevice, s), "H2D vout");
+    if (!st && acc && whole)
+        st = cuda_check(ctx, cudaMemcpyAsync(ctx->scratch_out.p, vout, bytes, cudaMemcpyHostToDevice, s), "H2D vout");
     if (st) return st;
-    if (bytes < kChunkBytes || ctx->nrows < kChunks) {
+    if (whole) {
         st = launch_applyh(ctx, ctx->scratch_in.p, ctx->scratch_out.p, nb, prec, acc, s);
         if (!st) st = cuda_check(ctx, cudaMemcpyAsync(vout, ctx->scratch_out.p, bytes, cudaMemcpyDeviceToHost, s), "D2H vout");
         if (!st) st = cuda_check(ctx, cudaStreamSynchronize(s), "applyh sync");
@@ -1472,22 +1492,34 @@ int applyh_on(bsg_ctx *ctx, const void *vin, void *vout, int nb, int prec, int f
     if (!ctx->copy_stream &&
         (st = cuda_check(ctx, cudaStreamCreateWithFlags(&ctx->copy_stream, cudaStreamNonBlocking), "copy stream")))
         return st;
-    while ((int)ctx->chunk_ev.size() < kChunks) {
+    while ((int)ctx->chunk_ev.size() <= kChunks) {
         cudaEvent_t e = nullptr;
         if ((st = cuda_check(ctx, cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "chunk event"))) return st;
         ctx->chunk_ev.push_back(e);
     }
+    // an accumulating call's vout comes in on the copy stream (after s, whose
+    // earlier work may write it), each chunk's part before its launch and
+    // beside the launch before
+    const size_t esz = (size_t)nb * (prec == BSG_PREC_FP32 ? 4 : 8);
+    if (acc && !(st = cuda_check(ctx, cudaEventRecord(ctx->chunk_ev[kChunks], s), "chunk event record")))
+        st = cuda_check(ctx, cudaStreamWaitEvent(ctx->copy_stream, ctx->chunk_ev[kChunks], 0), "chunk wait");
+    const std::vector<int64_t> cut = chunk_states(ctx);
     for (int c = 0; c < kChunks && !st; ++c) {
+        const size_t off = (size_t)cut[c] * esz, len = (size_t)(cut[c + 1] - cut[c]) * esz;
+        if (acc && len) {
+            st = cuda_check(ctx, cudaMemcpyAsync((char *)ctx->scratch_out.p + off, (const char *)vout + off, len,
+                                                 cudaMemcpyHostToDevice, ctx->copy_stream),
+                            "H2D vout chunk");
+            if (!st) st = cuda_check(ctx, cudaEventRecord(ctx->chunk_ev[kChunks], ctx->copy_stream), "chunk event record");
+            if (!st) st = cuda_check(ctx, cudaStreamWaitEvent(s, ctx->chunk_ev[kChunks], 0), "chunk wait");
+        }
         t_chunk = c;
-        st = launch_applyh(ctx, ctx->scratch_in.p, ctx->scratch_out.p, nb, prec, acc, s, chunk_lookup);
+        if (!st) st = launch_applyh(ctx, ctx->scratch_in.p, ctx->scratch_out.p, nb, prec, acc, s, chunk_lookup);
         if (!st) st = cuda_check(ctx, cudaEventRecord(ctx->chunk_ev[c], s), "chunk event record");
     }
     t_chunk = 0;
-    const ChunkTiles *ct = any_chunk_tiles(ctx);
-    if (!st && !ct) st = set_err(ctx, BSG_ERR_NOMEM, "bsg_applyh: chunked row tiles");
-    const size_t esz = (size_t)nb * (prec == BSG_PREC_FP32 ? 4 : 8);
     for (int c = 0; c < kChunks && !st; ++c) {
-        const size_t off = (size_t)ct->s0[c] * esz, len = (size_t)(ct->s0[c + 1] - ct->s0[c]) * esz;
+        const size_t off = (size_t)cut[c] * esz, len = (size_t)(cut[c + 1] - cut[c]) * esz;
         st = cuda_check(ctx, cudaStreamWaitEvent(ctx->copy_stream, ctx->chunk_ev[c], 0), "chunk wait");
         if (!st && len)
             st = cuda_check(ctx, cudaMemcpyAsync((char *)vout + off, (const char *)ctx->scratch_out.p + off, len,

@@ -160,12 +160,11 @@ struct TileSet {
 
 // row tiles cut into row-range chunks (host-pointer applyH copies each
 // chunk's output out while the next chunks run): one owned buffer, chunk c's
-// tiles at [start[c], start[c+1]) in longest-processing-time order, its
-// states [s0[c], s0[c+1]); view[c] points into the buffer (not owned)
+// tiles at [start[c], start[c+1]) in longest-processing-time order; view[c]
+// points into the buffer (not owned)
 struct ChunkTiles {
     DevBuf buf;
     std::vector<int32_t> start;
-    std::vector<int64_t> s0;
     std::vector<TileSet> view;
 };
 
