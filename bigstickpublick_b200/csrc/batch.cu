@@ -1,8 +1,10 @@
 // Batched Hamiltonians: many independent systems of uneven dimension.
 //
-// bsg_batch_applyh  one persistent launch applies every system's H: CTAs pull
-//                   (system, row tile) work items, heaviest first, from an
-//                   atomic counter; the tile body is the single-system one
+// bsg_batch_applyh  the systems with jump groups in one launch, one CTA per
+//                   (system, row), heaviest first, with the single-system row
+//                   body (rowgroup.cuh); the others in one persistent launch:
+//                   CTAs pull (system, row tile) work items, heaviest first,
+//                   from an atomic counter, with the single-system tile body
 //                   (applyh_tile.cuh).  No device-side waits.
 // bsg_batch_lanczos lock-step scalar Lanczos over all systems in the
 //                   reference's order: alpha and W -= alpha v_i first, then
