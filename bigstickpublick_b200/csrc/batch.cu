@@ -30,6 +30,9 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <memory>
+#include <mutex>
+#include <new>
 #include <numeric>
 #include <type_traits>
 #include <vector>
@@ -44,9 +47,20 @@ struct BatchSys {
     RowArgs a;
     GroupArgs g;        // grouped contexts, with their shared-memory layout
     int32_t parts[2], accel[2], bufel[2];
+};
+// a system's vectors in one call.  The descriptors above are written when the
+// batch's items are built and only read by the launches; what differs from call
+// to call lies in that call's own table, so that calls on several streams or
+// host threads do not meet.
+struct BatchVec {
     const void *vin;
     void *vout;
 };
+// device table of a call: the persistent kernel's work counter, then the vectors
+constexpr size_t kBatchVecOff = 16;
+// a batch keeps this many tables: so many calls may be in flight before one
+// waits (on its stream) for the launches of an earlier call
+constexpr int kBatchTables = 8;
 struct BatchItem {
     int32_t sys;
     int32_t tile;
@@ -72,8 +86,9 @@ struct BChunk {
 constexpr int kChunk = 2048;
 
 template <typename T, int ITEMS, bool SACC = false>
-__device__ __forceinline__ void rows_batch_body(const BatchSys *__restrict__ sys, const BatchItem *__restrict__ items,
-                                                int nitems, int *__restrict__ counter, int mstride) {
+__device__ __forceinline__ void rows_batch_body(const BatchSys *__restrict__ sys, const BatchVec *__restrict__ vec,
+                                                const BatchItem *__restrict__ items, int nitems,
+                                                int *__restrict__ counter, int mstride) {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ int s_item;
     const int warp = threadIdx.x >> 5;
@@ -87,16 +102,18 @@ __device__ __forceinline__ void rows_batch_body(const BatchSys *__restrict__ sys
         if (it >= nitems) return;
         const BatchItem w = items[it];
         const BatchSys *S = sys + w.sys;
-        row_tile<T, 1, ITEMS, false, kStore, false, SACC>(S->a, S->a.tiles[w.tile], (const T *)S->vin, (T *)S->vout, 1, 0, Mw, part);
+        row_tile<T, 1, ITEMS, false, kStore, false, SACC>(S->a, S->a.tiles[w.tile], (const T *)vec[w.sys].vin,
+                                                          (T *)vec[w.sys].vout, 1, 0, Mw, part);
         __syncthreads();
     }
 }
 
 template <typename T, int ITEMS>
 __global__ void __launch_bounds__(kWarps * 32) k_rows_batch(const BatchSys *__restrict__ sys,
+                                                            const BatchVec *__restrict__ vec,
                                                             const BatchItem *__restrict__ items, int nitems,
                                                             int *__restrict__ counter, int mstride) {
-    rows_batch_body<T, ITEMS>(sys, items, nitems, counter, mstride);
+    rows_batch_body<T, ITEMS>(sys, vec, items, nitems, counter, mstride);
 }
 
 // FP32: capped at 40 registers so that 6 CTAs of 256 threads stay resident
@@ -111,15 +128,17 @@ __global__ void __launch_bounds__(kWarps * 32) k_rows_batch(const BatchSys *__re
 // pick them).
 template <int ITEMS>
 __global__ void __launch_bounds__(kWarps * 32, ITEMS >= 4 ? 8 : 6) k_rows_batch_f32(const BatchSys *__restrict__ sys,
+                                                                   const BatchVec *__restrict__ vec,
                                                                    const BatchItem *__restrict__ items, int nitems,
                                                                    int *__restrict__ counter, int mstride) {
-    rows_batch_body<float, ITEMS, (ITEMS >= 2)>(sys, items, nitems, counter, mstride);
+    rows_batch_body<float, ITEMS, (ITEMS >= 2)>(sys, vec, items, nitems, counter, mstride);
 }
 
 // grouped contexts: one CTA per (system, row), heaviest first; the system's
 // descriptor is staged in shared memory
 template <typename T>
 __global__ void __launch_bounds__(256, 4) k_rowgroup_batch(const BatchSys *__restrict__ sys,
+                                                            const BatchVec *__restrict__ vec,
                                                             const BatchItem *__restrict__ items) {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ BatchSys S;
@@ -129,8 +148,8 @@ __global__ void __launch_bounds__(256, 4) k_rowgroup_batch(const BatchSys *__res
     __syncthreads();
     const Tile t = S.a.tiles[w.tile];
     constexpr int P = sizeof(T) == 8 ? 1 : 0;
-    row_group<T, 1, kStore>(S.a, S.g, S.parts[P], t.row, t.npos, (const T *)S.vin, 1, (T *)S.vout, nullptr,
-                            reinterpret_cast<T *>(smem), S.accel[P], S.bufel[P]);
+    row_group<T, 1, kStore>(S.a, S.g, S.parts[P], t.row, t.npos, (const T *)vec[w.sys].vin, 1, (T *)vec[w.sys].vout,
+                            nullptr, reinterpret_cast<T *>(smem), S.accel[P], S.bufel[P]);
 }
 
 template <typename T, int ITEMS>
@@ -375,12 +394,18 @@ struct bsg_batch {
     int items = 4;            // ITEMS of the batched row kernel (tile width 32*items)
     int ctas_per_sm = 4;
     int mstride = 4;
-    DevBuf sys, work, counter, workg;
+    DevBuf sys, work, workg;
     int nitems = 0;
     int nitemsg = 0;          // (system, row) items of the grouped contexts
     int nsm = 148;
     bool tuned = false;
-    std::vector<BatchSys> hsys;   // host copy of the descriptors
+    // the calls' tables, taken in turn; an event after the launches of the last
+    // call that used each
+    DevBuf ring;
+    size_t ring_stride = 0;
+    std::mutex ring_mu;
+    int ring_at = 0;
+    cudaEvent_t ring_ev[kBatchTables] = {};
 };
 
 namespace {
@@ -444,25 +469,36 @@ int build_items(bsg_batch *b, int items) {
         return berr(b, st, c0->last_error);
     b->nitems = (int)sorted.size();
     b->nitemsg = (int)sortedg.size();
-    b->hsys = std::move(sys);
     b->items = items;
     return BSG_OK;
 }
 
-// point every system's vin/vout at the given vectors, on the stream of the
-// launches that read them
-int set_vectors(bsg_batch *b, const void *const *vin, void *const *vout, cudaStream_t s) {
-    for (int k = 0; k < b->n; ++k) {
-        b->hsys[k].vin = vin[k];
-        b->hsys[k].vout = vout[k];
+// the host image of a call's table (null: no memory)
+std::unique_ptr<unsigned char[]> call_table(const bsg_batch *b, const void *const *vin, void *const *vout, size_t &bytes) {
+    bytes = kBatchVecOff + sizeof(BatchVec) * (size_t)b->n;
+    std::unique_ptr<unsigned char[]> t(new (std::nothrow) unsigned char[bytes]());
+    for (int k = 0; t && k < b->n; ++k) {
+        const BatchVec v{vin[k], vout[k]};
+        std::memcpy(t.get() + kBatchVecOff + sizeof(BatchVec) * (size_t)k, &v, sizeof v);
     }
-    if (cudaMemcpyAsync(b->sys.p, b->hsys.data(), sizeof(BatchSys) * b->n, cudaMemcpyHostToDevice, s) != cudaSuccess)
-        return berr(b, BSG_ERR_CUDA, "batch descriptor upload failed");
+    return t;
+}
+
+// the same on the device for as long as the caller's buffer lives, written
+// before the function returns
+int place_table(bsg_batch *b, DevBuf &d, const void *const *vin, void *const *vout) {
+    size_t bytes = 0;
+    const auto t = call_table(b, vin, vout, bytes);
+    const int st = t ? dev_alloc(b->ctx[0], d, bytes) : BSG_ERR_NOMEM;
+    if (st) return berr(b, st, "batch vector table: no memory");
+    if (cudaMemcpyAsync(d.p, t.get(), bytes, cudaMemcpyHostToDevice, b->stream) != cudaSuccess ||
+        cudaStreamSynchronize(b->stream) != cudaSuccess)
+        return berr(b, BSG_ERR_CUDA, "batch vector table upload failed");
     return BSG_OK;
 }
 
 template <typename T>
-int launch_batch_group(bsg_batch *b, cudaStream_t s) {
+int launch_batch_group(bsg_batch *b, const void *table, cudaStream_t s) {
     if (b->nitemsg == 0) return BSG_OK;
     size_t smem = 0;
     for (bsg_ctx *c : b->ctx)
@@ -471,7 +507,9 @@ int launch_batch_group(bsg_batch *b, cudaStream_t s) {
     cudaError_t e = smem > kGroupSmemMax ? cudaErrorInvalidValue
                                          : cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGroupSmemMax);
     if (e == cudaSuccess) {
-        kern<<<(unsigned)b->nitemsg, 256, smem, s>>>((const BatchSys *)b->sys.p, (const BatchItem *)b->workg.p);
+        kern<<<(unsigned)b->nitemsg, 256, smem, s>>>((const BatchSys *)b->sys.p,
+                                                       (const BatchVec *)((const char *)table + kBatchVecOff),
+                                                       (const BatchItem *)b->workg.p);
         e = cudaGetLastError();
     }
     if (e != cudaSuccess) return berr(b, BSG_ERR_CUDA, std::string("batched applyH: ") + cudaGetErrorString(e));
@@ -479,37 +517,39 @@ int launch_batch_group(bsg_batch *b, cudaStream_t s) {
 }
 
 template <typename T, int ITEMS>
-int launch_batch_t(bsg_batch *b, cudaStream_t s) {
-    if (const int st = launch_batch_group<T>(b, s)) return st;
+int launch_batch_t(bsg_batch *b, void *table, cudaStream_t s) {
+    if (const int st = launch_batch_group<T>(b, table, s)) return st;
     if (b->nitems == 0) return BSG_OK;
     const size_t smem = align16(sizeof(float) * (size_t)kWarps * b->mstride) + sizeof(T) * (size_t)kWarps * 32 * ITEMS;
     auto kern = batch_rows_kernel<T, ITEMS>();
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e == cudaSuccess) e = cudaMemsetAsync(b->counter.p, 0, sizeof(int), s);
+    if (e == cudaSuccess) e = cudaMemsetAsync(table, 0, sizeof(int), s);
     if (e == cudaSuccess) {
         const int grid = std::max(1, std::min(b->nitems, b->nsm * b->ctas_per_sm));
-        kern<<<grid, kWarps * 32, smem, s>>>((const BatchSys *)b->sys.p, (const BatchItem *)b->work.p,
-                                                                b->nitems, (int *)b->counter.p, b->mstride);
+        kern<<<grid, kWarps * 32, smem, s>>>((const BatchSys *)b->sys.p,
+                                             (const BatchVec *)((const char *)table + kBatchVecOff),
+                                             (const BatchItem *)b->work.p, b->nitems, (int *)table, b->mstride);
         e = cudaGetLastError();
     }
     if (e != cudaSuccess) return berr(b, BSG_ERR_CUDA, std::string("batched applyH: ") + cudaGetErrorString(e));
     return BSG_OK;
 }
 
-int launch_batch(bsg_batch *b, int prec, cudaStream_t s) {
+// table: the call's own (place_table's layout), in use until the launches end
+int launch_batch(bsg_batch *b, int prec, void *table, cudaStream_t s) {
     if (prec == BSG_PREC_FP32) {
         switch (b->items) {
-        case 1: return launch_batch_t<float, 1>(b, s);
-        case 2: return launch_batch_t<float, 2>(b, s);
-        case 8: return launch_batch_t<float, 8>(b, s);
-        default: return launch_batch_t<float, 4>(b, s);
+        case 1: return launch_batch_t<float, 1>(b, table, s);
+        case 2: return launch_batch_t<float, 2>(b, table, s);
+        case 8: return launch_batch_t<float, 8>(b, table, s);
+        default: return launch_batch_t<float, 4>(b, table, s);
         }
     }
     switch (b->items) {
-    case 1: return launch_batch_t<double, 1>(b, s);
-    case 2: return launch_batch_t<double, 2>(b, s);
-    case 8: return launch_batch_t<double, 8>(b, s);
-    default: return launch_batch_t<double, 4>(b, s);
+    case 1: return launch_batch_t<double, 1>(b, table, s);
+    case 2: return launch_batch_t<double, 2>(b, table, s);
+    case 8: return launch_batch_t<double, 8>(b, table, s);
+    default: return launch_batch_t<double, 4>(b, table, s);
     }
 }
 
@@ -564,12 +604,15 @@ int bsg_batch_create(int n, const bsg_tables *const *tables, const bsg_config *c
         if (cudaGetDeviceProperties(&prop, b->device) == cudaSuccess) b->nsm = prop.multiProcessorCount;
         if (cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking) != cudaSuccess) st = BSG_ERR_CUDA;
     }
-    if (!st) st = dev_alloc(b->ctx[0], b->counter, sizeof(int) * 4);
+    if (!st) {
+        b->ring_stride = (kBatchVecOff + sizeof(BatchVec) * (size_t)n + 255) & ~(size_t)255;
+        st = dev_alloc(b->ctx[0], b->ring, b->ring_stride * kBatchTables);
+    }
+    for (int k = 0; k < kBatchTables && !st; ++k)
+        if (cudaEventCreateWithFlags(&b->ring_ev[k], cudaEventDisableTiming) != cudaSuccess) st = BSG_ERR_CUDA;
     if (!st) st = build_items(b, 4);
     if (st) {
-        for (bsg_ctx *c : b->ctx) bsg_destroy(c);
-        if (b->stream) cudaStreamDestroy(b->stream);
-        delete b;
+        bsg_batch_destroy(b);
         return st;
     }
     *out = b;
@@ -583,7 +626,9 @@ int bsg_batch_destroy(bsg_batch *b) {
     dev_free(b->sys);
     dev_free(b->work);
     dev_free(b->workg);
-    dev_free(b->counter);
+    dev_free(b->ring);
+    for (cudaEvent_t e : b->ring_ev)
+        if (e) cudaEventDestroy(e);
     for (bsg_ctx *c : b->ctx) bsg_destroy(c);
     if (b->stream) cudaStreamDestroy(b->stream);
     delete b;
@@ -622,10 +667,30 @@ int bsg_batch_system(const bsg_batch *b, int s, bsg_ctx **ctx) {
 int bsg_batch_applyh(bsg_batch *b, const void *const *vin, void *const *vout, int prec, void *stream) {
     if (!b || !vin || !vout || (prec != BSG_PREC_FP32 && prec != BSG_PREC_FP64)) return BSG_ERR_ARG;
     cudaSetDevice(b->device);
-    int st = set_vectors(b, vin, vout, (cudaStream_t)stream);
-    if (st) return st;
     // stream: the caller's cudaStream_t; NULL is the legacy default stream
-    return launch_batch(b, prec, (cudaStream_t)stream);
+    cudaStream_t s = (cudaStream_t)stream;
+    // a graph would copy the table from host memory that is gone when it runs
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
+        cudaGetLastError();
+        return berr(b, BSG_ERR_CUDA, "bsg_batch_applyh cannot run while the stream is captured");
+    }
+    size_t bytes = 0;
+    const auto t = call_table(b, vin, vout, bytes);
+    if (!t) return berr(b, BSG_ERR_NOMEM, "bsg_batch_applyh: no host memory");
+    std::lock_guard<std::mutex> lock(b->ring_mu);
+    const int k = b->ring_at;
+    b->ring_at = (k + 1) % kBatchTables;
+    void *table = (char *)b->ring.p + b->ring_stride * (size_t)k;
+    // after the launches that last read this place, on whatever stream; the
+    // copy from pageable memory has left `t` when the call returns
+    cudaError_t e = cudaStreamWaitEvent(s, b->ring_ev[k], 0);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(table, t.get(), bytes, cudaMemcpyHostToDevice, s);
+    if (e != cudaSuccess) return berr(b, BSG_ERR_CUDA, std::string("batch vector table: ") + cudaGetErrorString(e));
+    const int st = launch_batch(b, prec, table, s);
+    e = cudaEventRecord(b->ring_ev[k], s);
+    if (!st && e != cudaSuccess) return berr(b, BSG_ERR_CUDA, std::string("batch event: ") + cudaGetErrorString(e));
+    return st;
 }
 
 // autotuner: time the batched matvec for each tile width and CTA residency,
@@ -633,7 +698,7 @@ int bsg_batch_applyh(bsg_batch *b, const void *const *vin, void *const *vout, in
 int bsg_batch_autotune(bsg_batch *b, int *items_out, int *ctas_out, double *best_ms_out) {
     if (!b) return BSG_ERR_ARG;
     cudaSetDevice(b->device);
-    DevBuf x, y;
+    DevBuf x, y, tab;
     bsg_ctx *c0 = b->ctx[0];
     int st;
     if ((st = dev_alloc(c0, x, sizeof(float) * b->total)) || (st = dev_alloc(c0, y, sizeof(float) * b->total))) {
@@ -656,14 +721,14 @@ int bsg_batch_autotune(bsg_batch *b, int *items_out, int *ctas_out, double *best
     // timed launches per candidate
     const int cand_items[] = {1, 2, 4, 8};
     const int cand_ctas[] = {4, 8};
+    st = place_table(b, tab, vi.data(), vo.data());
     for (int it : cand_items) {
-        if ((st = build_items(b, it))) break;
-        if ((st = set_vectors(b, vi.data(), vo.data(), b->stream))) break;
+        if (st || (st = build_items(b, it))) break;
         for (int cps : cand_ctas) {
             b->ctas_per_sm = cps;
-            launch_batch(b, BSG_PREC_FP32, b->stream);
+            launch_batch(b, BSG_PREC_FP32, tab.p, b->stream);
             cudaEventRecord(e0, b->stream);
-            for (int r = 0; r < 3; ++r) launch_batch(b, BSG_PREC_FP32, b->stream);
+            for (int r = 0; r < 3; ++r) launch_batch(b, BSG_PREC_FP32, tab.p, b->stream);
             cudaEventRecord(e1, b->stream);
             cudaEventSynchronize(e1);
             float ms = 0;
@@ -679,6 +744,7 @@ int bsg_batch_autotune(bsg_batch *b, int *items_out, int *ctas_out, double *best
     cudaEventDestroy(e1);
     dev_free(x);
     dev_free(y);
+    dev_free(tab);
     if (st) return st;
     b->ctas_per_sm = bc;
     if ((st = build_items(b, bi))) return st;
@@ -729,7 +795,7 @@ int bsg_batch_lanczos(bsg_batch *b, const bsg_lanczos_params *p, double *evals, 
         partsz += (int64_t)(niter + 1) * nch;
         sqsz += nch;
     }
-    DevBuf hist, X, Y, W, part, coef, sqp, ab, itd, chd, lzd, fl;
+    DevBuf hist, X, Y, W, part, coef, sqp, ab, itd, chd, lzd, fl, tab;
     int st;
     size_t fr = 0, tot = 0;
     cudaMemGetInfo(&fr, &tot);
@@ -793,7 +859,7 @@ int bsg_batch_lanczos(bsg_batch *b, const bsg_lanczos_params *p, double *evals, 
             vi[s] = (const char *)X.p + (size_t)esz * b->off[s];
             vo[s] = (char *)Y.p + (size_t)esz * b->off[s];
         }
-        st = set_vectors(b, vi.data(), vo.data(), b->stream);
+        st = place_table(b, tab, vi.data(), vo.data());
     }
     if (!st && cudaMemsetAsync(itd.p, 0, sizeof(int), s0) != cudaSuccess) st = BSG_ERR_CUDA;
     if (!st && cudaMemsetAsync(fl.p, 0, 16 * (size_t)n, s0) != cudaSuccess) st = BSG_ERR_CUDA;
@@ -814,7 +880,7 @@ int bsg_batch_lanczos(bsg_batch *b, const bsg_lanczos_params *p, double *evals, 
                 k_bpack<float><<<G, 256, 0, s0>>>((const BLz *)lzd.p, (const BChunk *)chd.p, nchunks, itp, (float *)X.p);
             else
                 k_bpack<double><<<G, 256, 0, s0>>>((const BLz *)lzd.p, (const BChunk *)chd.p, nchunks, itp, (double *)X.p);
-            int lst = launch_batch(b, p->matvec_prec, s0);
+            int lst = launch_batch(b, p->matvec_prec, tab.p, s0);
             const BLz *Lc = (const BLz *)lzd.p;
             BLz *Lm = (BLz *)lzd.p;
             const BChunk *Cc = (const BChunk *)chd.p;
@@ -931,7 +997,7 @@ int bsg_batch_lanczos(bsg_batch *b, const bsg_lanczos_params *p, double *evals, 
     if (graph) cudaGraphDestroy(graph);
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
-    DevBuf *bs[] = {&hist, &X, &Y, &W, &part, &coef, &sqp, &ab, &itd, &chd, &lzd, &fl};
+    DevBuf *bs[] = {&hist, &X, &Y, &W, &part, &coef, &sqp, &ab, &itd, &chd, &lzd, &fl, &tab};
     for (DevBuf *x : bs) dev_free(*x);
     return st;
 }

@@ -332,7 +332,9 @@ int  bsg_apply1b(bsg_ctx *ctx, const bsg_density_tables *dt, const double *ppot,
  *      (the reference runs one per process).  bsg_batch_applyh applies all of
  *      them in one persistent launch whose CTAs pull (system, row tile) work
  *      items heaviest first; vin[s]/vout[s] are device pointers of dim_s
- *      elements, launched on cuda_stream (NULL: the legacy default stream).  bsg_batch_lanczos runs lock-step scalar Lanczos on all
+ *      elements, launched on cuda_stream (NULL: the legacy default stream;
+ *      calls on several streams or host threads may be in flight together, a
+ *      capturing stream gets BSG_ERR_CUDA).  bsg_batch_lanczos runs lock-step scalar Lanczos on all
  *      systems for exactly p->niter iterations (uniform pivots, full
  *      classical Gram-Schmidt reorthogonalization) with each iteration
  *      captured once as a CUDA graph and replayed; evals[s*nkeep + k];
