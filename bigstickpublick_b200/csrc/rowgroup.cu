@@ -121,19 +121,37 @@ GroupShape group_shape(const bsg_ctx *ctx, int esize, int nv) {
     return r;
 }
 
-// Single vectors, odd blocks and blocks on long rows always; on short rows the
-// row-tile kernel, which takes the whole block in one walk, stays the better
-// one where a 16-byte load covers half the block or less (sd 6p6n: FP32 nb = 8
-// 151 us against 159, FP64 nb = 4 152 against 165, but nb = 16 381 / 1106
-// against 349 / 858), and on rows of a slice or two from one such load on (pf
-// 5p2n, rows of 17: FP64 nb = 8 1.28 ms against 1.98; sd 3p4n FP32 nb = 4 21
-// against 23 us).
+// The row-tile kernel takes a whole block in one walk, the jump groups nb / NV
+// walks, so which is faster depends on the block and the rows.  Both timed on one
+// B200 over sd 1p1n ... 8p8n and pf 1p1n ... 8p1n, 3p6n; figures are row-tile time /
+// jump-group time.
+//  - Long rows (one part): the groups, 1.37 - 1.92 for single and paired vectors,
+//    at least 1.13 for FP32 and 1.03 for FP64 blocks (rows of 390 to 3,500).
+//  - Rows of at most half a slice, more of them than CTAs fit at once, one or two
+//    vectors: the row tiles.  There a CTA is mostly start and end, of eight warps
+//    here as there (FP64 one vector 0.81 - 1.00, two 0.77 - 0.94; FP32 two 0.79 -
+//    0.95; FP32 one 0.90 - 0.98 where the second wave is half empty at best, sd 5p1n
+//    ... 7p2n, but 1.07 - 1.21 beyond).
+//  - Odd blocks and those below one 16-byte load: the groups, 0.96 and more there
+//    too (the row tiles split odd blocks: 1.1 - 9).
+//  - Powers of two from one 16-byte load up, short rows: a median of 64 and less
+//    the row tiles (FP64 nb = 8 down to 0.46, FP32 nb = 16 the same) but for pairs;
+//    above, the row tiles at two loads (FP32 nb = 8 0.94 - 1.07, FP64 nb = 4 0.90 -
+//    1.03) and, where the rows fill the chip twice, at four (pf 4p3n ... 6p3n: FP64
+//    nb = 8 0.95 - 0.97, FP32 nb = 16 0.97 - 0.99; pf 3p3n, 1,140 rows, 1.02; sd
+//    1.01 - 1.14); the groups elsewhere (FP32 nb = 4 1.05 - 1.5, FP64 nb = 16 1.09 -
+//    2).  Spaces of some dozen rows scatter: sd 2p6n loses at FP32 nb = 16 (0.78)
+//    what sd 2p8n gains (1.26).
 bool group_takes(const bsg_ctx *ctx, int nb, int prec) {
     if (!ctx->grouped) return false;
+    if (group_shape(ctx, prec, 1).parts == 1) return true;
+    constexpr int64_t wave = 148 * 4;   // CTAs of eight one-warp parts
     const int nv = 16 / prec;
-    if (nb < nv || (nb & (nb - 1)) || nb > 16 || group_shape(ctx, prec, 1).parts == 1) return true;
+    if (nb <= 2 && ctx->median_rowlen <= 16 && ctx->nrows > wave)
+        return nb == 1 && prec == BSG_PREC_FP32 && 2 * ctx->nrows > 3 * wave;
+    if (nb < nv || (nb & (nb - 1)) || nb > 16) return true;
     if (ctx->median_rowlen <= 64) return nb == 2;
-    return nb != 2 * nv;
+    return nb != 2 * nv && (nb != 4 * nv || ctx->nrows <= 2 * wave);
 }
 
 int launch_rowgroup(bsg_ctx *ctx, const void *vin, void *vout, int nb, int prec, int accumulate, cudaStream_t s,
