@@ -1235,7 +1235,21 @@ int derive(bsg_ctx *ctx, const bsg_tables *t, const bsg_tables3 *t3, bool do_upl
     a.ld_cpn = ld;
     a.ncpn = (int32_t)cpn32.size();
     const GroupSource gs{nops, nop_maxin, nptr_all, spe_ptr, pn};
-    return group_eligible(ctx, gs, pack32) ? build_groups(ctx, gs, nthr) : BSG_OK;
+    if (!group_eligible(ctx, gs, pack32)) return BSG_OK;
+    // the groups come on top of the row tiles' tables, which are complete:
+    // where they do not fit in memory or in their indexes, the row tiles take
+    // the context
+    int st_g;
+    try {
+        st_g = build_groups(ctx, gs, nthr);
+    } catch (const std::bad_alloc &) {
+        st_g = BSG_ERR_NOMEM;
+    }
+    if (st_g != BSG_ERR_NOMEM && st_g != BSG_ERR_UNSUPPORTED) return st_g;
+    free_groups(ctx);
+    ctx->last_error.clear();
+    ctx->last_status = BSG_OK;
+    return BSG_OK;
 }
 
 void free_ctx(bsg_ctx *ctx) {

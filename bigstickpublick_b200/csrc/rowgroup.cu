@@ -355,6 +355,10 @@ int build_groups(bsg_ctx *ctx, const GroupSource &S, int nthr) {
     return BSG_OK;
 }
 
-void free_groups(bsg_ctx *ctx) { dev_free(ctx->g_buf); }
+void free_groups(bsg_ctx *ctx) {
+    dev_free(ctx->g_buf);
+    ctx->group = GroupArgs{};
+    ctx->grouped = false;
+}
 
 }  // namespace bsg

@@ -22,6 +22,7 @@ struct GroupSource {
 };
 // whether the context takes the jump-group kernel
 bool group_eligible(bsg_ctx *ctx, const GroupSource &S, bool pack32);
+// BSG_ERR_NOMEM, BSG_ERR_UNSUPPORTED (or std::bad_alloc): the context has none
 int build_groups(bsg_ctx *ctx, const GroupSource &S, int nthr);
 void free_groups(bsg_ctx *ctx);
 
