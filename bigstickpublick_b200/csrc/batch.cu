@@ -798,8 +798,13 @@ int bsg_batch_lanczos(bsg_batch *b, const bsg_lanczos_params *p, double *evals, 
     DevBuf hist, X, Y, W, part, coef, sqp, ab, itd, chd, lzd, fl, tab;
     int st;
     size_t fr = 0, tot = 0;
+    const size_t need = (size_t)histsz * 8 + (size_t)b->total * (2 * esz + 8);
     cudaMemGetInfo(&fr, &tot);
-    if ((size_t)histsz * 8 + (size_t)b->total * (2 * esz + 8) > fr)
+    if (need > fr) {
+        pool_trim(b->device);
+        cudaMemGetInfo(&fr, &tot);
+    }
+    if (need > fr)
         return berr(b, BSG_ERR_NOMEM, "bsg_batch_lanczos: histories do not fit in device memory");
     if ((st = dev_alloc(c0, hist, 8 * (size_t)histsz)) || (st = dev_alloc(c0, X, (size_t)esz * b->total)) ||
         (st = dev_alloc(c0, Y, (size_t)esz * b->total)) || (st = dev_alloc(c0, W, 8 * (size_t)b->total)) ||

@@ -19,6 +19,7 @@
 #include <numeric>
 #include <set>
 #include <thread>
+#include <mutex>
 #include <unordered_map>
 
 #include "bsg_internal.h"
@@ -48,6 +49,12 @@ int dev_alloc(bsg_ctx *ctx, DevBuf &b, size_t bytes) {
     dev_free(b);
     if (bytes == 0) bytes = 16;
     cudaError_t e = cudaMalloc(&b.p, bytes);
+    if (e == cudaErrorMemoryAllocation) {
+        // cudaMalloc cannot draw on what the scratch pool keeps
+        cudaGetLastError();
+        pool_trim(ctx->device);
+        e = cudaMalloc(&b.p, bytes);
+    }
     if (e != cudaSuccess) {
         b.p = nullptr;
         return cuda_check(ctx, e, "cudaMalloc");
@@ -69,25 +76,42 @@ int upload(bsg_ctx *ctx, DevBuf &b, const void *src, size_t bytes) {
     return BSG_OK;
 }
 
+namespace {
+// the scratch pool of a device, shared by its contexts
+struct DevicePool {
+    std::mutex mu;
+    cudaMemPool_t pool = nullptr;
+    int users = 0;   // contexts that have drawn on it
+};
+constexpr int kMaxDevices = 64;
+DevicePool g_pools[kMaxDevices];
+}  // namespace
+
 int pool_alloc(bsg_ctx *ctx, DevBuf &b, size_t bytes, cudaStream_t s) {
+    if (ctx->device < 0 || ctx->device >= kMaxDevices)
+        return set_err(ctx, BSG_ERR_UNSUPPORTED, "device ordinal out of range");
+    DevicePool &P = g_pools[ctx->device];
     {
-        std::lock_guard<std::mutex> lock(ctx->pool_mu);
-        if (!ctx->pool) {
+        std::lock_guard<std::mutex> lock(P.mu);
+        if (!P.pool) {
             cudaMemPoolProps props{};
             props.allocType = cudaMemAllocationTypePinned;
             props.location.type = cudaMemLocationTypeDevice;
             props.location.id = ctx->device;
-            int st = cuda_check(ctx, cudaMemPoolCreate(&ctx->pool, &props), "cudaMemPoolCreate");
+            int st = cuda_check(ctx, cudaMemPoolCreate(&P.pool, &props), "cudaMemPoolCreate");
             if (st) {
-                ctx->pool = nullptr;
+                P.pool = nullptr;
                 return st;
             }
             uint64_t keep = kPoolKeep;
-            cudaMemPoolSetAttribute(ctx->pool, cudaMemPoolAttrReleaseThreshold, &keep);
+            cudaMemPoolSetAttribute(P.pool, cudaMemPoolAttrReleaseThreshold, &keep);
         }
+        if (!ctx->uses_pool) ++P.users;
+        ctx->uses_pool = true;
     }
     b.bytes = bytes ? bytes : 16;
-    const int st = cuda_check(ctx, cudaMallocFromPoolAsync(&b.p, b.bytes, ctx->pool, s), "cudaMallocFromPoolAsync");
+    // the pool lives as long as a context that uses it
+    const int st = cuda_check(ctx, cudaMallocFromPoolAsync(&b.p, b.bytes, P.pool, s), "cudaMallocFromPoolAsync");
     if (st) b = DevBuf{};
     return st;
 }
@@ -98,9 +122,39 @@ int pool_upload(bsg_ctx *ctx, DevBuf &b, const void *src, size_t bytes, cudaStre
     return cuda_check(ctx, cudaMemcpyAsync(b.p, src, bytes, cudaMemcpyHostToDevice, s), "upload");
 }
 
-void pool_free(DevBuf &b, cudaStream_t s) {
-    if (b.p) cudaFreeAsync(b.p, s);
-    b = DevBuf{};
+void pool_free(std::initializer_list<DevBuf *> bufs, cudaStream_t s) {
+    size_t bytes = 0;
+    for (DevBuf *b : bufs) {
+        if (b->p) {
+            cudaFreeAsync(b->p, s);
+            bytes += b->bytes;
+        }
+        *b = DevBuf{};
+    }
+    // what lies above the pool's threshold goes back to the device at the
+    // stream's next synchronization: here, not at some later call
+    if (bytes > kPoolKeep) cudaStreamSynchronize(s);
+}
+
+void pool_trim(int device) {
+    if (device < 0 || device >= kMaxDevices) return;
+    DevicePool &P = g_pools[device];
+    std::lock_guard<std::mutex> lock(P.mu);
+    if (!P.pool) return;
+    // frees count as done once the host has seen their streams end
+    if (cudaDeviceSynchronize() != cudaSuccess || cudaMemPoolTrimTo(P.pool, 0) != cudaSuccess) cudaGetLastError();
+}
+
+// a context leaves its device's pool; the last one takes it down
+static void pool_leave(bsg_ctx *ctx) {
+    if (!ctx->uses_pool) return;
+    ctx->uses_pool = false;
+    DevicePool &P = g_pools[ctx->device];
+    std::lock_guard<std::mutex> lock(P.mu);
+    if (--P.users == 0) {
+        cudaMemPoolDestroy(P.pool);
+        P.pool = nullptr;
+    }
 }
 
 void build_tile_list(const bsg_ctx *ctx, int tp, std::vector<Tile> &tiles) {
@@ -1268,8 +1322,7 @@ void free_ctx(bsg_ctx *ctx) {
     ctx->chunk_tiles.clear();
     for (cudaEvent_t e : ctx->chunk_ev) cudaEventDestroy(e);
     ctx->chunk_ev.clear();
-    if (ctx->pool) cudaMemPoolDestroy(ctx->pool);
-    ctx->pool = nullptr;
+    pool_leave(ctx);
     if (ctx->copy_stream) cudaStreamDestroy(ctx->copy_stream);
     ctx->copy_stream = nullptr;
     if (ctx->ev0) cudaEventDestroy(ctx->ev0);

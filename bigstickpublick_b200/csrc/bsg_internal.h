@@ -4,8 +4,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <initializer_list>
 #include <map>
-#include <mutex>
 #include <string>
 #include <vector>
 
@@ -222,11 +222,7 @@ struct bsg_ctx {
     std::map<int, bsg::ChunkTiles> chunk_tiles;
     cudaStream_t copy_stream = nullptr;
     std::vector<cudaEvent_t> chunk_ev;
-    // stream-ordered scratch of the state calls (adjoint, densities): the
-    // context's own pool, which keeps up to kPoolKeep between calls and goes
-    // with the context
-    std::mutex pool_mu;
-    cudaMemPool_t pool = nullptr;
+    bool uses_pool = false;   // counted among the users of its device's scratch pool
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
 };
 
@@ -236,11 +232,15 @@ int cuda_check(bsg_ctx *ctx, cudaError_t e, const char *what);
 int dev_alloc(bsg_ctx *ctx, DevBuf &b, size_t bytes);
 void dev_free(DevBuf &b);
 int upload(bsg_ctx *ctx, DevBuf &b, const void *src, size_t bytes);
-// stream-ordered scratch from the context's pool; freed on the same stream
+// stream-ordered scratch of the state calls (adjoint, densities), freed on the
+// same stream: one pool per device, which keeps up to kPoolKeep between calls, for
+// all contexts together, and goes with the last context that used it
 constexpr uint64_t kPoolKeep = (uint64_t)1 << 30;
 int pool_alloc(bsg_ctx *ctx, DevBuf &b, size_t bytes, cudaStream_t s);
 int pool_upload(bsg_ctx *ctx, DevBuf &b, const void *src, size_t bytes, cudaStream_t s);
-void pool_free(DevBuf &b, cudaStream_t s);
+void pool_free(std::initializer_list<DevBuf *> bufs, cudaStream_t s);
+// gives back what the pool keeps (waits for the device)
+void pool_trim(int device);
 const TileSet *get_tiles(bsg_ctx *ctx, int tp);
 // row tiles of width tp in longest-processing-time order (host list)
 void build_tile_list(const bsg_ctx *ctx, int tp, std::vector<Tile> &tiles);

@@ -195,9 +195,7 @@ int grad_many(bsg_ctx *const *ctxs, int nsys, const double *const *evecs, int ns
     }
     bsg_ctx *c0 = ctxs[0];
     DevBuf psi, tmp, acc, out, descb, itemb, nnb, nnrb;
-    auto cleanup = [&]() {
-        for (DevBuf *b : {&psi, &tmp, &acc, &out, &descb, &itemb, &nnb, &nnrb}) pool_free(*b, s);
-    };
+    auto cleanup = [&]() { pool_free({&psi, &tmp, &acc, &out, &descb, &itemb, &nnb, &nnrb}, s); };
     int st;
     if (nstates == 1) rows = false;   // the same layout
     if ((st = pool_alloc(c0, psi, sizeof(double) * (size_t)npsi, s)) ||

@@ -699,6 +699,10 @@ extern "C" int bsg_lanczos(bsg_ctx *ctx, const bsg_lanczos_params *p, const doub
                   (size_t)L.n * L.nb * (L.prec == 4 ? 4 : 8);
     size_t fr = 0, tot = 0;
     cudaMemGetInfo(&fr, &tot);
+    if (need > fr) {
+        pool_trim(ctx->device);
+        cudaMemGetInfo(&fr, &tot);
+    }
     if (need > fr) return set_err(ctx, BSG_ERR_NOMEM, "bsg_lanczos: history does not fit in device memory");
     const int G = dot_grid(L.n);
     const int ktmp = std::max(L.nb, pp.nkeep + std::max(pp.nthick_add, 0) + 1);

@@ -268,6 +268,10 @@ int  bsg_grad(bsg_ctx *ctx, const double *evecs, int nstates,
  * basis state side by side) */
 int  bsg_grad_rows(bsg_ctx *ctx, const double *evecs, int nstates,
               double *dpp, double *dnn, double *dpn, double *dspe_p, double *dspe_n);
+/*      Device scratch of this call and of bsg_density1b comes from a pool of the
+ *      device, which keeps at most 1 GiB between calls for all contexts together
+ *      and gives it back when the last context that used it is destroyed, or when
+ *      another allocation of this library needs it. */
 /*      All states in one launch; every label's sum is accumulated exactly (to
  *      2^-64) in 128-bit fixed point with integer atomics, so the result is
  *      bitwise repeatable and independent of how the work is split. */

@@ -1,0 +1,70 @@
+"""Device memory that gradients and densities keep between calls: at most 1 GiB for
+all contexts of the device, given back to other allocations of the library when
+they need it, and to the device with the last context.
+
+Memory is compared with 64 MiB of allowance (allocation granularity, tile lists)."""
+import numpy as np
+import pytest
+
+from bigstickpublick_b200 import model
+
+pytestmark = pytest.mark.gpu
+
+GIB, SLACK = 1 << 30, 64 << 20
+
+
+def _free():
+    import torch
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    return torch.cuda.mem_get_info()[0]
+
+
+@pytest.fixture(scope="module")
+def tables():
+    return model.build_tables(model.pf_model(4, 4, seed=5))   # dim 1,963,461: 15.7 MB a state
+
+
+def test_kept_memory_is_bounded_and_given_back(tables):
+    import torch
+    from bigstickpublick_b200.engine import Hamiltonian
+    t = tables
+    hams = [Hamiltonian(t) for _ in range(4)]
+    v = np.zeros((t.dim, 32))
+    v[np.arange(32) * 1000, np.arange(32)] = 1.0
+    hams[0].density1b(v[:, :2])   # kernels and events in place
+    base = _free()
+    for h in hams:
+        h.density1b(v)   # 0.5 GB of scratch each
+    assert base - _free() <= GIB + SLACK
+    # a call that needs more (1.3 GB, two layouts of 40 states) keeps no more
+    w = np.zeros((t.dim, 40))
+    w[np.arange(40) * 1000, np.arange(40)] = 1.0
+    hams[0].grad(w)
+    kept = base - torch.cuda.mem_get_info()[0]   # no synchronization in between
+    assert kept <= GIB + SLACK
+    # what is kept serves the library's other allocations: vectors of a host
+    # applyH (2 x 126 MB), a Lanczos history (12 columns, 188 MB and work space)
+    hams[0].density1b(v)
+    hog = torch.empty(_free() - (96 << 20), dtype=torch.uint8, device="cuda")
+    try:
+        y = hams[1].applyh(np.ones((t.dim, 8)))
+        assert np.isfinite(y).all()
+    finally:
+        del hog
+    hams[0].density1b(v)
+    hog = torch.empty(_free() - (96 << 20), dtype=torch.uint8, device="cuda")
+    try:
+        e, _, _ = hams[2].lanczos(nkeep=1, niter=12, matvec_prec=8, fixed_iter=True)
+        assert np.isfinite(e).all()
+    finally:
+        del hog
+    for h in hams:
+        h.close()
+    hams = None
+    h = Hamiltonian(t)
+    before = _free()
+    h.density1b(v)
+    assert before - _free() > 256 << 20   # kept while a user lives
+    h.close()
+    assert _free() >= before - SLACK
