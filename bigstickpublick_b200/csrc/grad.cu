@@ -39,13 +39,13 @@ __global__ void k_fix_to_double(const unsigned long long *__restrict__ acc, doub
         out[i] = fix_value(acc + 2 * i);
 }
 
-// [dim x ns] row-major -> column-major; a warp takes 32 states, whose lines
-// stay in L1 between the columns
-__global__ void k_rows_to_cols(const double *__restrict__ x, int64_t dim, int ns, double *__restrict__ y) {
+// [n x ns] row-major -> n rows of columns ld apart; a warp takes 32 states, whose
+// lines stay in L1 between the columns
+__global__ void k_rows_to_cols(const double *__restrict__ x, int64_t n, int ns, double *__restrict__ y, int64_t ld) {
     const int lane = threadIdx.x & 31;
-    for (int64_t r = ((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5) * 32 + lane; r < dim;
+    for (int64_t r = ((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5) * 32 + lane; r < n;
          r += (int64_t)gridDim.x * blockDim.x)
-        for (int k = 0; k < ns; ++k) y[(int64_t)k * dim + r] = __ldg(x + r * ns + k);
+        for (int k = 0; k < ns; ++k) y[(int64_t)k * ld + r] = __ldg(x + r * ns + k);
 }
 
 // three CTAs to an SM: at 128 registers (two) five states of sd 6p6n took 1.72 ms
@@ -107,6 +107,8 @@ constexpr int kGradStates = 5;
 constexpr size_t kGradSmem = 113 * 1024;
 // and enough CTAs for the chip: of a small system each state has its own
 constexpr int64_t kGradCtas = 148 * 4;
+// row-major states on their way to columns: 64 MB at a time
+constexpr int64_t kGradPiece = (int64_t)8 << 20;
 
 template <int NS>
 cudaError_t launch_items(const DevBuf &descb, const GradItem *items, size_t n, int mstride, cudaStream_t s) {
@@ -198,8 +200,13 @@ int grad_many(bsg_ctx *const *ctxs, int nsys, const double *const *evecs, int ns
     auto cleanup = [&]() { pool_free({&psi, &tmp, &acc, &out, &descb, &itemb, &nnb, &nnrb}, s); };
     int st;
     if (nstates == 1) rows = false;   // the same layout
+    // row-major states come in so many basis states at a time, so that they do
+    // not lie on the device twice
+    const int64_t piece = std::max<int64_t>(1, kGradPiece / nstates);
+    int64_t maxdim = 0;
+    for (int s2 = 0; s2 < nsys; ++s2) maxdim = std::max(maxdim, ctxs[s2]->dim);
     if ((st = pool_alloc(c0, psi, sizeof(double) * (size_t)npsi, s)) ||
-        (rows && (st = pool_alloc(c0, tmp, sizeof(double) * (size_t)npsi, s))) ||
+        (rows && (st = pool_alloc(c0, tmp, sizeof(double) * (size_t)(std::min(piece, maxdim) * nstates), s))) ||
         (st = pool_alloc(c0, acc, 16 * (size_t)nacc, s)) || (st = pool_alloc(c0, out, sizeof(double) * (size_t)nacc, s))) {
         cleanup();
         return fail(st, "device allocation: " + c0->last_error);
@@ -238,14 +245,18 @@ int grad_many(bsg_ctx *const *ctxs, int nsys, const double *const *evecs, int ns
         return fail(st, "upload: " + c0->last_error);
     }
     cudaError_t e = cudaSuccess;
-    for (int s2 = 0; s2 < nsys && e == cudaSuccess; ++s2)
-        e = cudaMemcpyAsync((double *)(rows ? tmp.p : psi.p) + psi_off[s2], evecs[s2],
-                            sizeof(double) * ctxs[s2]->dim * nstates, cudaMemcpyHostToDevice, s);
-    for (int s2 = 0; rows && s2 < nsys && e == cudaSuccess; ++s2) {
+    for (int s2 = 0; s2 < nsys && e == cudaSuccess; ++s2) {
         const int64_t dim = ctxs[s2]->dim;
-        k_rows_to_cols<<<(unsigned)std::min<int64_t>((dim + 255) / 256, 148 * 8), 256, 0, s>>>(
-            (const double *)tmp.p + psi_off[s2], dim, nstates, (double *)psi.p + psi_off[s2]);
-        e = cudaGetLastError();
+        double *to = (double *)psi.p + psi_off[s2];
+        if (!rows) e = cudaMemcpyAsync(to, evecs[s2], sizeof(double) * dim * nstates, cudaMemcpyHostToDevice, s);
+        for (int64_t r = 0; rows && r < dim && e == cudaSuccess; r += piece) {
+            const int64_t n = std::min(piece, dim - r);
+            e = cudaMemcpyAsync(tmp.p, evecs[s2] + r * nstates, sizeof(double) * n * nstates, cudaMemcpyHostToDevice, s);
+            if (e != cudaSuccess) break;
+            k_rows_to_cols<<<(unsigned)std::min<int64_t>((n + 255) / 256, 148 * 8), 256, 0, s>>>(
+                (const double *)tmp.p, n, nstates, to + r, dim);
+            e = cudaGetLastError();
+        }
     }
     if (e == cudaSuccess) e = cudaMemsetAsync(acc.p, 0, acc.bytes, s);
     cudaEvent_t e0 = nullptr, e1 = nullptr;
