@@ -963,7 +963,7 @@ int derive(bsg_ctx *ctx, const bsg_tables *t, const bsg_tables3 *t3, bool do_upl
     auto nrec_of = [&](int32_t id) -> int64_t { return nptr_all[nops[id].ptr_base + nops[id].nout]; };
     // ---- sliced records: per operator, output positions in slices of 32;
     // a slice holds its longest position's count of 32-record rows, record k
-    // of lane l at row k (padding rows hold {0, 0} and are never read)
+    // of lane l at row k (shorter positions: see the unused places below)
     std::vector<int2> sell_all;
     std::vector<int32_t> slice_off_all;
     // 32-bit copy when every input position, (b,d) index and hmatnn label fits
@@ -974,7 +974,7 @@ int derive(bsg_ctx *ctx, const bsg_tables *t, const bsg_tables3 *t3, bool do_upl
     // labels do not fit, the NN entries stay zero and FP64 keeps the 8-byte
     // records (ctx->rec32_nn)
     const int64_t nmatnn_all = t->nmatnn + (three ? t3->nmatnnn : 0);
-    const bool pack32 = ctx->max_rowlen <= 65535 && max_nbd_all <= 32768;
+    const bool pack32 = ctx->max_rowlen <= 65536 && max_nbd_all <= 32768;
     const bool nn32 = pack32 && nmatnn_all <= 32768;
     ctx->rec32_nn = nn32;
     std::vector<uint32_t> sell32_all;
@@ -1018,13 +1018,16 @@ int derive(bsg_ctx *ctx, const bsg_tables *t, const bsg_tables3 *t3, bool do_upl
                 slice_off_all[op.slice_base + sl] = (int32_t)off;
                 const size_t row0 = (size_t)(op.sell_base + off);
                 // unused places: the jump-group kernel reads them as a record
-                // of a position that it keeps zero (one past the operator's
-                // input positions, one past the longest row); the row-tile
-                // kernels count records and never read them
+                // of a position (one past the operator's input positions, one
+                // past the longest row) and, in a PN operator, of a label (one
+                // past its own) that it keeps zero; the row-tile kernels count
+                // records and never read them (nor are they read where the
+                // fields are too narrow: group_eligible)
                 const int32_t zero_pos = op.kind == 1 ? nop_maxin[o] + 1 : ctx->max_rowlen;
+                const uint32_t zero32 = ((uint32_t)zero_pos & 0xffffu) | ((uint32_t)(op.kind == 1 ? op.nbd : 0) & 0x7fffu) << 16;
                 for (size_t q = row0; q < row0 + (size_t)32 * width; ++q) {
                     sell_all[q] = make_int2(zero_pos, 0);
-                    if (pack32) sell32_all[q] = (uint32_t)zero_pos;
+                    if (pack32) sell32_all[q] = zero32;
                 }
                 for (int l = 0; l < 32 && 32 * sl + l < op.nout; ++l)
                     for (int32_t k = ptr[32 * sl + l]; k < ptr[32 * sl + l + 1]; ++k) {
