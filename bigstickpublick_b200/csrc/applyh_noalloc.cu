@@ -72,6 +72,15 @@ thread_local bsg::TileSet t_static_tiles;
 const bsg::TileSet *static_tiles(bsg_ctx *ctx, int tp) {
     auto it = ctx->tiles.find(tp);
     if (it != ctx->tiles.end()) return &it->second;
+    // a host applyH in row ranges has cached its own list, range after range in
+    // one buffer
+    auto ct = ctx->chunk_tiles.find(tp);
+    if (ct != ctx->chunk_tiles.end()) {
+        t_static_tiles.buf.p = ct->second.buf.p;
+        t_static_tiles.buf.bytes = ct->second.buf.bytes;
+        t_static_tiles.ntiles = ct->second.start.back();
+        return &t_static_tiles;
+    }
     std::vector<bsg::Tile> tiles;
     bsg::build_tile_list(ctx, tp, tiles);
     const size_t bytes = tiles.size() * sizeof(bsg::Tile);
