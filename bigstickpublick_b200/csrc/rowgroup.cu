@@ -125,15 +125,17 @@ GroupShape group_shape(const bsg_ctx *ctx, int esize, int nv) {
 // walks, so which is faster depends on the block and the rows.  Both timed on one
 // B200 over sd 1p1n ... 8p8n and pf 1p1n ... 8p1n, 3p6n; figures are row-tile time /
 // jump-group time.
-//  - Long rows (one part): the groups, 1.37 - 1.92 for single and paired vectors,
-//    at least 1.13 for FP32 and 1.03 for FP64 blocks (rows of 390 to 3,500).
-//  - Rows of at most half a slice, more of them than CTAs fit at once, one or two
-//    vectors: the row tiles.  There a CTA is mostly start and end, of eight warps
-//    here as there (FP64 one vector 0.81 - 1.00, two 0.77 - 0.94; FP32 two 0.79 -
-//    0.95; FP32 one 0.90 - 0.98 where the second wave is half empty at best, sd 5p1n
-//    ... 7p2n, but 1.07 - 1.21 beyond).
-//  - Odd blocks and those below one 16-byte load: the groups, 0.96 and more there
-//    too (the row tiles split odd blocks: 1.1 - 9).
+//  - Single vectors: the groups, 1.02 - 2.6.  On rows of a few positions, more of
+//    them than CTAs fit at once, the row tiles would be the faster by a few us (sd
+//    5p1n ... 7p2n FP64 0.81 - 0.88, FP32 0.90 - 0.98), but a batch of such systems
+//    is 1.3 (FP64) to 2 times (FP32) faster on the groups, and a member has the bits
+//    of the same system alone.
+//  - Long rows (one part): the groups, at least 1.13 for FP32 and 1.03 for FP64
+//    blocks (rows of 390 to 3,500).
+//  - Pairs on rows of at most half a slice, more of them than CTAs fit at once: the
+//    row tiles (0.77 - 0.95).  There a CTA is mostly start and end.
+//  - Odd blocks and those below one 16-byte load: the groups (the row tiles split
+//    odd blocks: 0.97 - 9).
 //  - Powers of two from one 16-byte load up, short rows: a median of 64 and less
 //    the row tiles (FP64 nb = 8 down to 0.46, FP32 nb = 16 the same) but for pairs;
 //    above, the row tiles at two loads (FP32 nb = 8 0.94 - 1.07, FP64 nb = 4 0.90 -
@@ -144,11 +146,10 @@ GroupShape group_shape(const bsg_ctx *ctx, int esize, int nv) {
 //    what sd 2p8n gains (1.26).
 bool group_takes(const bsg_ctx *ctx, int nb, int prec) {
     if (!ctx->grouped) return false;
-    if (group_shape(ctx, prec, 1).parts == 1) return true;
+    if (nb == 1 || group_shape(ctx, prec, 1).parts == 1) return true;
     constexpr int64_t wave = 148 * 4;   // CTAs of eight one-warp parts
     const int nv = 16 / prec;
-    if (nb <= 2 && ctx->median_rowlen <= 16 && ctx->nrows > wave)
-        return nb == 1 && prec == BSG_PREC_FP32 && 2 * ctx->nrows > 3 * wave;
+    if (nb == 2 && ctx->median_rowlen <= 16 && ctx->nrows > wave) return false;
     if (nb < nv || (nb & (nb - 1)) || nb > 16) return true;
     if (ctx->median_rowlen <= 64) return nb == 2;
     return nb != 2 * nv && (nb != 4 * nv || ctx->nrows <= 2 * wave);

@@ -1,7 +1,6 @@
 """The rule that sends applyH to the jump groups or to the row tiles, on both
 sides of its lines, against the oracle: rows of a few positions, fewer and more
-of them than CTAs fit at once and than one and a half times as many (sd 4p2n,
-6p2n, pf 3p1n); rows of about a hundred, below and above twice as many (pf 3p3n,
+of them than CTAs fit at once (sd 4p2n, 6p2n, pf 3p1n); rows of about a hundred, below and above twice as many (pf 3p3n,
 4p3n); blocks of one, two and four 16-byte loads.
 
 Tolerances as in test_rowgroup_gpu.py: FP64 1e-12 of the largest output, FP32
