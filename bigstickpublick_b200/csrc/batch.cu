@@ -517,8 +517,7 @@ int launch_batch_group(bsg_batch *b, const void *table, cudaStream_t s) {
 }
 
 template <typename T, int ITEMS>
-int launch_batch_t(bsg_batch *b, void *table, cudaStream_t s) {
-    if (const int st = launch_batch_group<T>(b, table, s)) return st;
+int launch_tiles_t(bsg_batch *b, void *table, cudaStream_t s) {
     if (b->nitems == 0) return BSG_OK;
     const size_t smem = align16(sizeof(float) * (size_t)kWarps * b->mstride) + sizeof(T) * (size_t)kWarps * 32 * ITEMS;
     auto kern = batch_rows_kernel<T, ITEMS>();
@@ -535,22 +534,28 @@ int launch_batch_t(bsg_batch *b, void *table, cudaStream_t s) {
     return BSG_OK;
 }
 
-// table: the call's own (place_table's layout), in use until the launches end
-int launch_batch(bsg_batch *b, int prec, void *table, cudaStream_t s) {
+// the members without jump groups.  table: the call's own (place_table's
+// layout), in use until the launches end
+int launch_tiles(bsg_batch *b, int prec, void *table, cudaStream_t s) {
     if (prec == BSG_PREC_FP32) {
         switch (b->items) {
-        case 1: return launch_batch_t<float, 1>(b, table, s);
-        case 2: return launch_batch_t<float, 2>(b, table, s);
-        case 8: return launch_batch_t<float, 8>(b, table, s);
-        default: return launch_batch_t<float, 4>(b, table, s);
+        case 1: return launch_tiles_t<float, 1>(b, table, s);
+        case 2: return launch_tiles_t<float, 2>(b, table, s);
+        case 8: return launch_tiles_t<float, 8>(b, table, s);
+        default: return launch_tiles_t<float, 4>(b, table, s);
         }
     }
     switch (b->items) {
-    case 1: return launch_batch_t<double, 1>(b, table, s);
-    case 2: return launch_batch_t<double, 2>(b, table, s);
-    case 8: return launch_batch_t<double, 8>(b, table, s);
-    default: return launch_batch_t<double, 4>(b, table, s);
+    case 1: return launch_tiles_t<double, 1>(b, table, s);
+    case 2: return launch_tiles_t<double, 2>(b, table, s);
+    case 8: return launch_tiles_t<double, 8>(b, table, s);
+    default: return launch_tiles_t<double, 4>(b, table, s);
     }
+}
+
+int launch_batch(bsg_batch *b, int prec, void *table, cudaStream_t s) {
+    const int st = prec == BSG_PREC_FP32 ? launch_batch_group<float>(b, table, s) : launch_batch_group<double>(b, table, s);
+    return st ? st : launch_tiles(b, prec, table, s);
 }
 
 }  // namespace
@@ -693,8 +698,9 @@ int bsg_batch_applyh(bsg_batch *b, const void *const *vin, void *const *vout, in
     return st;
 }
 
-// autotuner: time the batched matvec for each tile width and CTA residency,
-// keep the fastest (vectors are scratch, fp32)
+// autotuner: time the persistent launch for each tile width and CTA residency,
+// keep the fastest (vectors are scratch, fp32).  The jump groups' launch has no
+// choice to make: a batch whose members all have groups keeps its setting.
 int bsg_batch_autotune(bsg_batch *b, int *items_out, int *ctas_out, double *best_ms_out) {
     if (!b) return BSG_ERR_ARG;
     cudaSetDevice(b->device);
@@ -716,38 +722,46 @@ int bsg_batch_autotune(bsg_batch *b, int *items_out, int *ctas_out, double *best
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
     double best = 1e300;
-    int bi = 4, bc = 4;
-    // 2 CTAs per SM never won on the measured batches; one warm-up and three
-    // timed launches per candidate
+    int bi = b->items, bc = b->ctas_per_sm;
+    // mean of three launches after one warm-up
+    auto timed = [&](auto launch) -> double {
+        launch();
+        cudaEventRecord(e0, b->stream);
+        for (int r = 0; r < 3; ++r) launch();
+        cudaEventRecord(e1, b->stream);
+        cudaEventSynchronize(e1);
+        float ms = 0;
+        cudaEventElapsedTime(&ms, e0, e1);
+        return ms / 3;
+    };
+    // 2 CTAs per SM never won on the measured batches
     const int cand_items[] = {1, 2, 4, 8};
     const int cand_ctas[] = {4, 8};
     st = place_table(b, tab, vi.data(), vo.data());
     for (int it : cand_items) {
-        if (st || (st = build_items(b, it))) break;
+        if (st || b->nitems == 0 || (st = build_items(b, it))) break;
         for (int cps : cand_ctas) {
             b->ctas_per_sm = cps;
-            launch_batch(b, BSG_PREC_FP32, tab.p, b->stream);
-            cudaEventRecord(e0, b->stream);
-            for (int r = 0; r < 3; ++r) launch_batch(b, BSG_PREC_FP32, tab.p, b->stream);
-            cudaEventRecord(e1, b->stream);
-            cudaEventSynchronize(e1);
-            float ms = 0;
-            cudaEventElapsedTime(&ms, e0, e1);
-            if (ms / 3 < best) {
-                best = ms / 3;
+            const double ms = timed([&]() { launch_tiles(b, BSG_PREC_FP32, tab.p, b->stream); });
+            if (ms < best) {
+                best = ms;
                 bi = it;
                 bc = cps;
             }
         }
     }
+    if (!st && b->nitems) {
+        b->ctas_per_sm = bc;
+        st = build_items(b, bi);
+    }
+    // the whole call with that setting
+    if (!st) best = timed([&]() { launch_batch(b, BSG_PREC_FP32, tab.p, b->stream); });
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     dev_free(x);
     dev_free(y);
     dev_free(tab);
     if (st) return st;
-    b->ctas_per_sm = bc;
-    if ((st = build_items(b, bi))) return st;
     b->tuned = true;
     if (items_out) *items_out = bi;
     if (ctas_out) *ctas_out = bc;
