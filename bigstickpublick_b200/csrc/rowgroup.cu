@@ -15,10 +15,17 @@ namespace {
 
 // one CTA per row and NV of the block's vectors, heaviest rows first, a row's
 // vectors next to each other (they share the records and, where the vectors
-// are interleaved, the sectors); 64 registers a thread, so that 32 warps stay
-// resident per SM
-template <typename T, int NV, int OUT, bool BIG>
-__global__ void __launch_bounds__(BIG ? 1024 : 256, BIG ? 1 : 4)
+// are interleaved, the sectors).  FORM: up to 256 threads with 64 registers, so that
+// 32 warps stay resident per SM; up to 1024 threads; or, for single vectors on many
+// rows of a few positions, 256 threads with 40 registers and 48 warps: there a CTA
+// waits on one short chain of loads, and more rows at once outweigh the spills
+// (60 bytes at most).  Calls with 64 / 40 / 32 registers: sd 6p2n FP64 33.6 / 28.9 /
+// 30.7 us, FP32 29.7 / 25.6 / 27.0, pf 5p1n FP64 247 / 214 / 212, FP32 191 / 172 / 169;
+// but pf 3p2n (rows of 23) FP32 34.0 / 38.0 / 35.2, sd 4p2n (all rows at once anyway)
+// 24.5 / 25.6 / 28.1.
+enum RowForm { kSmallCta = 0, kBigCta = 1, kManyCtas = 2 };
+template <typename T, int NV, int OUT, int FORM>
+__global__ void __launch_bounds__(FORM == kBigCta ? 1024 : 256, FORM == kBigCta ? 1 : (FORM == kManyCtas ? 6 : 4))
     k_rowgroup(const RowArgs a, const GroupArgs g, const int parts, const T *__restrict__ vin, const int64_t ld,
                T *__restrict__ vout, const int accel, const int bufel, const int ngrp) {
     extern __shared__ __align__(16) unsigned char smem[];
@@ -27,6 +34,9 @@ __global__ void __launch_bounds__(BIG ? 1024 : 256, BIG ? 1 : 4)
     row_group<T, NV, OUT>(a, g, parts, t.row, t.npos, vin + v, ld, vout + v,
                           OUT == kColumns ? a.cols_out + v * a.cols_ld : nullptr, reinterpret_cast<T *>(smem), accel, bufel);
 }
+
+// CTAs of 256 threads and 64 registers that fit at once
+constexpr int64_t kGroupWave = 148 * 4;
 
 struct VKey {
     int32_t nop, aoff, coff;
@@ -48,7 +58,7 @@ __global__ void k_vrows(const RowArgs a, const VKey *__restrict__ key, const int
     }
 }
 
-template <typename T, int NV, int OUT, bool BIG>
+template <typename T, int NV, int OUT, int FORM>
 int launch_k(bsg_ctx *ctx, const GroupShape &sh, const T *vin, T *vout, int nb, cudaStream_t s, const TileSet *ts,
              double *cols) {
     RowArgs a = ctx->args;
@@ -56,7 +66,7 @@ int launch_k(bsg_ctx *ctx, const GroupShape &sh, const T *vin, T *vout, int nb, 
     a.ntiles = ts->ntiles;
     a.cols_out = cols;
     a.cols_ld = ctx->dim;
-    auto k = k_rowgroup<T, NV, OUT, BIG>;
+    auto k = k_rowgroup<T, NV, OUT, FORM>;
     // the attribute belongs to the function, not the context: set to the
     // limit once, so that contexts of different sizes do not undo one another's
     size_t &cur = ctx->smem_allowed[(const void *)k];
@@ -70,16 +80,22 @@ int launch_k(bsg_ctx *ctx, const GroupShape &sh, const T *vin, T *vout, int nb, 
     return cuda_check(ctx, cudaGetLastError(), "applyh kernel launch");
 }
 
+// rows of at most half a slice, more of them than CTAs of 64 registers fit at once
+bool many_short_rows(const bsg_ctx *ctx) { return ctx->median_rowlen <= 16 && ctx->nrows > kGroupWave; }
+
 template <typename T, int NV>
 int launch_v(bsg_ctx *ctx, const T *vin, T *vout, int nb, int accumulate, cudaStream_t s, const TileSet *ts, double *cols) {
     const GroupShape sh = group_shape(ctx, sizeof(T), NV);
-    auto big = [&](auto b) {
-        constexpr bool B = decltype(b)::value;
-        if (cols) return launch_k<T, NV, kColumns, B>(ctx, sh, vin, vout, nb, s, ts, cols);
-        if (accumulate) return launch_k<T, NV, kAccumulate, B>(ctx, sh, vin, vout, nb, s, ts, cols);
-        return launch_k<T, NV, kStore, B>(ctx, sh, vin, vout, nb, s, ts, cols);
+    auto go = [&](auto f) {
+        constexpr int F = decltype(f)::value;
+        if (cols) return launch_k<T, NV, kColumns, F>(ctx, sh, vin, vout, nb, s, ts, cols);
+        if (accumulate) return launch_k<T, NV, kAccumulate, F>(ctx, sh, vin, vout, nb, s, ts, cols);
+        return launch_k<T, NV, kStore, F>(ctx, sh, vin, vout, nb, s, ts, cols);
     };
-    return sh.threads > 256 ? big(std::true_type{}) : big(std::false_type{});
+    if (sh.threads > 256) return go(std::integral_constant<int, kBigCta>{});
+    if constexpr (NV == 1)
+        if (nb == 1 && many_short_rows(ctx)) return go(std::integral_constant<int, kManyCtas>{});
+    return go(std::integral_constant<int, kSmallCta>{});
 }
 
 template <typename T>
@@ -125,11 +141,10 @@ GroupShape group_shape(const bsg_ctx *ctx, int esize, int nv) {
 // walks, so which is faster depends on the block and the rows.  Both timed on one
 // B200 over sd 1p1n ... 8p8n and pf 1p1n ... 8p1n, 3p6n; figures are row-tile time /
 // jump-group time.
-//  - Single vectors: the groups, 1.02 - 2.6.  On rows of a few positions, more of
-//    them than CTAs fit at once, the row tiles would be the faster by a few us (sd
-//    5p1n ... 7p2n FP64 0.81 - 0.88, FP32 0.90 - 0.98), but a batch of such systems
-//    is 1.3 (FP64) to 2 times (FP32) faster on the groups, and a member has the bits
-//    of the same system alone.
+//  - Single vectors: the groups, 1.02 - 2.6 (0.93 - 1.1 on many rows of a few
+//    positions, sd 5p1n ... 7p2n FP64 with 48 warps to an SM; a batch of such systems
+//    is 1.3 - 2 times faster on the groups, and a member has the bits of the same
+//    system alone).
 //  - Long rows (one part): the groups, at least 1.13 for FP32 and 1.03 for FP64
 //    blocks (rows of 390 to 3,500).
 //  - Pairs on rows of at most half a slice, more of them than CTAs fit at once: the
@@ -147,12 +162,11 @@ GroupShape group_shape(const bsg_ctx *ctx, int esize, int nv) {
 bool group_takes(const bsg_ctx *ctx, int nb, int prec) {
     if (!ctx->grouped) return false;
     if (nb == 1 || group_shape(ctx, prec, 1).parts == 1) return true;
-    constexpr int64_t wave = 148 * 4;   // CTAs of eight one-warp parts
     const int nv = 16 / prec;
-    if (nb == 2 && ctx->median_rowlen <= 16 && ctx->nrows > wave) return false;
+    if (nb == 2 && many_short_rows(ctx)) return false;
     if (nb < nv || (nb & (nb - 1)) || nb > 16) return true;
     if (ctx->median_rowlen <= 64) return nb == 2;
-    return nb != 2 * nv && (nb != 4 * nv || ctx->nrows <= 2 * wave);
+    return nb != 2 * nv && (nb != 4 * nv || ctx->nrows <= 2 * kGroupWave);
 }
 
 int launch_rowgroup(bsg_ctx *ctx, const void *vin, void *vout, int nb, int prec, int accumulate, cudaStream_t s,
