@@ -183,7 +183,9 @@ struct bsg_ctx {
     int32_t median_rowlen = 0;
     int32_t max_nb = 16;
     int32_t pn_table_max = 512;   // bsg_config.pn_table_max
-    // raw tables on the device (byte-identical copies)
+    // the device arrays, all in `tables` (the buffers below are views of it):
+    // raw tables (byte-identical copies)
+    bsg::DevBuf tables;
     std::vector<bsg::DevBuf> raw;
     // derived
     bsg::DevBuf row_off, pp_ptr, nn_ptr, pn_ptr, spe_ptr, pp, nn, pn, spe, nops, nptr, pnrec, nnrec, bd, sell, slice_off;
