@@ -63,24 +63,14 @@ __device__ __forceinline__ double flip_sign(double x, unsigned bit31) {
     return __hiloint2double(__double2hiint(x) ^ (int)bit31, __double2loint(x));
 }
 
-// the warps of one part of a CTA
+// the warps of one part of a CTA: one warp, or all of the CTA (group_shape)
 struct Part {
     int id, g, w, lane;    // part, its warps, this warp among them
-    bool whole;            // the only part
     __device__ __forceinline__ void sync() const {
-        if (g == 1) {
+        if (g == 1)
             __syncwarp();
-        } else if (whole) {
+        else
             __syncthreads();
-        } else {
-            // at most 4 parts of several warps
-            switch (id) {
-            case 0: asm volatile("bar.sync 1, %0;" ::"r"(g * 32) : "memory"); break;
-            case 1: asm volatile("bar.sync 2, %0;" ::"r"(g * 32) : "memory"); break;
-            case 2: asm volatile("bar.sync 3, %0;" ::"r"(g * 32) : "memory"); break;
-            default: asm volatile("bar.sync 4, %0;" ::"r"(g * 32) : "memory"); break;
-            }
-        }
     }
 };
 
@@ -188,8 +178,10 @@ template <typename T, int NV> constexpr int kGroupJumps = sizeof(T) == 4 && NV =
 // One row, NV vectors (consecutive elements; ld elements between positions).
 // smem: per part acc[accel] and the staging buffer [bufel] (elements of T).
 // The row's work items lie in 8 slots; part p of P takes 8 / P of them and
-// keeps its own sums, added in part order at the end.  P depends on the
-// context alone, so every kernel adds in the same order.
+// keeps its own sums, added in part order at the end.  P follows from the
+// context, T and NV, and so do the jumps of a group, so the order of the sum is
+// fixed for these three (the single and the batched kernel share it); a block's
+// column, or a block on another base (which allows another NV), rounds otherwise.
 template <typename T, int NV, int OUT>
 __device__ __forceinline__ void row_group(const RowArgs &a, const GroupArgs &g, const int parts, const int row, const int len,
                                           const T *__restrict__ vin, const int64_t ld_, T *__restrict__ vout,
@@ -198,7 +190,6 @@ __device__ __forceinline__ void row_group(const RowArgs &a, const GroupArgs &g, 
     const int64_t ld = NV == 1 ? ld_ : (ld_ & ~(int64_t)(NV - 1));   // a multiple of NV
     Part pt;
     pt.lane = threadIdx.x & 31;
-    pt.whole = parts == 1;
     pt.g = (blockDim.x >> 5) / parts;
     pt.id = (threadIdx.x >> 5) / pt.g;
     pt.w = (threadIdx.x >> 5) - pt.id * pt.g;
