@@ -1562,9 +1562,9 @@ int applyh_on(bsg_ctx *ctx, const void *vin, void *vout, int nb, int prec, int f
     if (flags & BSG_DEVICE_PTRS) return launch_applyh(ctx, vin, vout, nb, prec, acc, s);
     // host pointers: copy in, apply, copy out (the drop-in path for vec1/vec2)
     const size_t bytes = (size_t)ctx->dim * nb * (prec == BSG_PREC_FP32 ? 4 : 8);
-    if (ctx->scratch_in.bytes < bytes) {
-        if ((st = dev_alloc(ctx, ctx->scratch_in, bytes)) || (st = dev_alloc(ctx, ctx->scratch_out, bytes))) return st;
-    }
+    // each by itself: a call that found room for one only has left the other empty
+    for (DevBuf *b : {&ctx->scratch_in, &ctx->scratch_out})
+        if (b->bytes < bytes && (st = dev_alloc(ctx, *b, bytes))) return st;
     const bool whole = !chunked(ctx, bytes, nb, prec);
     st = cuda_check(ctx, cudaMemcpyAsync(ctx->scratch_in.p, vin, bytes, cudaMemcpyHostToDevice, s), "H2D vin");
     if (!st && acc && whole)
