@@ -5,6 +5,7 @@
 #include <atomic>
 #include <cstdint>
 #include <new>
+#include <system_error>
 #include <thread>
 #include <vector>
 
@@ -38,8 +39,13 @@ void parallel_for(int64_t n, int64_t chunk, F fn, int max_threads = 32) {
             oom = true;   // reported to the caller below as an allocation failure
         }
     };
+    // fewer threads where the system gives no more: the chunks go round all the same
     std::vector<std::thread> th;
-    for (int k = 1; k < nt; ++k) th.emplace_back(work);
+    th.reserve((size_t)nt);
+    try {
+        for (int k = 1; k < nt; ++k) th.emplace_back(work);
+    } catch (const std::system_error &) {
+    }
     work();
     for (auto &x : th) x.join();
     if (oom) throw std::bad_alloc();
