@@ -100,8 +100,11 @@ __global__ void __launch_bounds__(kGradWarps * 32) k_grad_nn(const GradDesc *__r
 
 namespace {
 constexpr int kGradItems = 4;  // 128-position tiles
-// states in one pass over the records, at most: calls on sd 6p6n with 1, 2, 3
-// and 5, for five states 1.95, 1.78, 1.92, 1.72 ms, for two 0.92, then 0.81
+// states in one pass over the records, at most.  Whole calls with at most 3, 4 and 5:
+// pf 3p4n five states 10.4, 10.6, 9.3 ms, ten 20.1, 19.2, 17.8, twelve 22.9, 22.0, 22.0;
+// pf 3p3n five 2.53, 2.51, 2.31, ten 4.46, 4.39, 4.18; sd 6p6n five 1.69, 1.70, 1.57,
+// ten 3.03, 2.93, 2.81, eight 2.48, 2.33, 2.31; sd 5p5n five 1.31, 1.31, 1.21.  For 1,
+// 2, 3, 6 and 8 states 4 and 5 give the same groups or times within 2 %.
 constexpr int kGradStates = 5;
 // no more shared memory than leaves two CTAs on an SM
 constexpr size_t kGradSmem = 113 * 1024;

@@ -285,12 +285,13 @@ class _SystemView(Hamiltonian):
 
 
 class Batch:
-    """Many independent Hamiltonians (bsg_batch_*): one persistent launch
-    applies all of them; Lanczos runs lock-step with one captured CUDA graph
-    per iteration.
+    """Many independent Hamiltonians (bsg_batch_*): one launch applies those
+    with jump groups, one persistent launch the others; Lanczos runs lock-step
+    with one captured CUDA graph per iteration.
 
     tune_cache: JSON file mapping a batch signature to the autotuned
-    (tile width, CTAs per SM); read if present, written after autotuning."""
+    (tile width, CTAs per SM) of the persistent launch; read if present, written
+    after autotuning."""
 
     def __init__(self, tables_list, device=0, autotune=False, tune_cache=None):
         self.lib = _abi.gpu_lib()
@@ -366,11 +367,11 @@ class Batch:
         self._check(self.lib.bsg_batch_applyh(self.h, vi, vo, prec, C.c_void_p(s)), "bsg_batch_applyh")
 
     def grad(self, vecs):
-        """Adjoint gradients of every system in one launch (bsg_batch_grad):
+        """Adjoint gradients of every system in one call (bsg_batch_grad):
         vecs[s] dim_s x k eigenvectors of system s; returns a list of dicts
         of (k, nmat) arrays 'pp', 'nn', 'pn' (and 'spe_p', 'spe_n' for
         members with SPE bundles), bitwise equal to each member's own
-        Hamiltonian.grad, and sets self.grad_ms to the launch's device time."""
+        Hamiltonian.grad, and sets self.grad_ms to the launches' device time."""
         n = len(self.tables)
         if len(vecs) != n:
             raise ValueError("one eigenvector block per system")

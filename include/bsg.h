@@ -226,7 +226,11 @@ int  bsg_last_error(const bsg_ctx *ctx, char *buf, size_t len);
  *      for nb > 1.  Vectors of nb interleaved vectors: element (state s,
  *      vector v) at (s-1)*nb + v (src/bmodules_block.f90:19-22).
  *      prec: BSG_PREC_FP32 (float vectors, fp32 accumulation) or
- *      BSG_PREC_FP64 (double vectors, fp32 matrix elements promoted). ---- */
+ *      BSG_PREC_FP64 (double vectors, fp32 matrix elements promoted).
+ *      No atomics: the same call on the same vectors gives the same bits.  The
+ *      order of a sum follows from the context, prec, nb and whether vin is
+ *      aligned to 16 (8) bytes; a column of a block, or the same block on another
+ *      base, may round otherwise. ---- */
 int  bsg_applyh(bsg_ctx *ctx, const void *vin, void *vout, int nb, int prec, int flags);
 /* same on a caller-provided cudaStream_t (device pointers only) */
 int  bsg_applyh_stream(bsg_ctx *ctx, const void *vin, void *vout, int nb, int prec,
@@ -272,9 +276,11 @@ int  bsg_grad_rows(bsg_ctx *ctx, const double *evecs, int nstates,
  *      device, which keeps at most 1 GiB between calls for all contexts together
  *      and gives it back when the last context that used it is destroyed, or when
  *      another allocation of this library needs it. */
-/*      All states in one launch; every label's sum is accumulated exactly (to
- *      2^-64) in 128-bit fixed point with integer atomics, so the result is
- *      bitwise repeatable and independent of how the work is split. */
+/*      All states in one call.  The products of a label are added in FP64 inside
+ *      a fixed group (a warp's positions, 16 rows of an NN operator) and the
+ *      groups exactly (to 2^-64) in 128-bit fixed point with integer atomics, so
+ *      the result is bitwise repeatable and does not depend on how many states
+ *      or systems share a launch. */
 
 /* ---- one-body densities: replaces master_density1b_bundled
  *      (src/bdenslib1.f90:1506-1607), i.e. applyP1Bdenbundled_g and
@@ -334,8 +340,10 @@ int  bsg_apply1b(bsg_ctx *ctx, const bsg_density_tables *dt, const double *ppot,
 
 /* ---- batched systems: many independent Hamiltonians of uneven dimension
  *      (the reference runs one per process).  bsg_batch_applyh applies all of
- *      them in one persistent launch whose CTAs pull (system, row tile) work
- *      items heaviest first; vin[s]/vout[s] are device pointers of dim_s
+ *      them: the systems with jump groups in one launch with a CTA per (system,
+ *      row), the others (few long rows, or no PN bundles) in one persistent
+ *      launch whose CTAs pull (system, row tile) work items heaviest first;
+ *      vin[s]/vout[s] are device pointers of dim_s
  *      elements, launched on cuda_stream (NULL: the legacy default stream;
  *      calls on several streams or host threads may be in flight together, a
  *      capturing stream gets BSG_ERR_CUDA).  bsg_batch_lanczos runs lock-step scalar Lanczos on all
@@ -343,8 +351,10 @@ int  bsg_apply1b(bsg_ctx *ctx, const bsg_density_tables *dt, const double *ppot,
  *      classical Gram-Schmidt reorthogonalization) with each iteration
  *      captured once as a CUDA graph and replayed; evals[s*nkeep + k];
  *      evecs NULL or n host pointers of dim_s*nkeep doubles.  The tile width
- *      and CTA residency of the batched kernel come from bsg_batch_autotune
- *      (timed on the device) or bsg_batch_set_tuning. ---- */
+ *      and CTA residency of the persistent launch come from bsg_batch_autotune
+ *      (timed on the device; a batch whose systems all have jump groups keeps
+ *      its setting, and best_ms is the time of a call either way) or
+ *      bsg_batch_set_tuning. ---- */
 typedef struct bsg_batch bsg_batch;
 int  bsg_batch_create(int n, const bsg_tables *const *tables, const bsg_config *cfg, bsg_batch **out);
 int  bsg_batch_destroy(bsg_batch *b);
@@ -356,12 +366,12 @@ int  bsg_batch_autotune(bsg_batch *b, int *items, int *ctas_per_sm, double *best
 int  bsg_batch_set_tuning(bsg_batch *b, int items, int ctas_per_sm);
 int  bsg_batch_lanczos(bsg_batch *b, const bsg_lanczos_params *p, double *evals, double *const *evecs,
                        bsg_report *rep);
-/* adjoint gradients of every system of the batch in one launch over all
- * (system, state, row tile) items (the per-system bsg_grad of each member,
- * bitwise equal to it): evecs[s] host fp64 dim_s x nstates column-major;
+/* adjoint gradients of every system of the batch, in launches over all systems:
+ * (system, states, row tile) items, and (system, state, rows of an NN operator)
+ * ones (the per-system bsg_grad of each member, bitwise equal to it): evecs[s] host fp64 dim_s x nstates column-major;
  * dpp[s], dnn[s], dpn[s] host fp64 [nstates x nmat*_s] (state-major), and
  * dspe_p[s] / dspe_n[s] for members with SPE bundles (arrays may be NULL).
- * kernel_ms (may be NULL): device time of the launch. */
+ * kernel_ms (may be NULL): device time of the launches. */
 int  bsg_batch_grad(bsg_batch *b, const double *const *evecs, int nstates, double *const *dpp,
                     double *const *dnn, double *const *dpn, double *const *dspe_p, double *const *dspe_n,
                     double *kernel_ms);
