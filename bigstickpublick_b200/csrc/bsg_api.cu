@@ -77,41 +77,38 @@ int upload(bsg_ctx *ctx, DevBuf &b, const void *src, size_t bytes) {
 }
 
 namespace {
-// the scratch pool of a device, shared by its contexts
-struct DevicePool {
+// the contexts of a device that have a scratch pool, the last used at the end
+struct DevicePools {
     std::mutex mu;
-    cudaMemPool_t pool = nullptr;
-    int users = 0;   // contexts that have drawn on it
+    std::vector<bsg_ctx *> users;
 };
 constexpr int kMaxDevices = 64;
-DevicePool g_pools[kMaxDevices];
+DevicePools g_pools[kMaxDevices];
 }  // namespace
 
 int pool_alloc(bsg_ctx *ctx, DevBuf &b, size_t bytes, cudaStream_t s) {
     if (ctx->device < 0 || ctx->device >= kMaxDevices)
         return set_err(ctx, BSG_ERR_UNSUPPORTED, "device ordinal out of range");
-    DevicePool &P = g_pools[ctx->device];
     {
+        DevicePools &P = g_pools[ctx->device];
         std::lock_guard<std::mutex> lock(P.mu);
-        if (!P.pool) {
+        if (!ctx->pool) {
             cudaMemPoolProps props{};
             props.allocType = cudaMemAllocationTypePinned;
             props.location.type = cudaMemLocationTypeDevice;
             props.location.id = ctx->device;
-            int st = cuda_check(ctx, cudaMemPoolCreate(&P.pool, &props), "cudaMemPoolCreate");
+            int st = cuda_check(ctx, cudaMemPoolCreate(&ctx->pool, &props), "cudaMemPoolCreate");
             if (st) {
-                P.pool = nullptr;
+                ctx->pool = nullptr;
                 return st;
             }
             uint64_t keep = kPoolKeep;
-            cudaMemPoolSetAttribute(P.pool, cudaMemPoolAttrReleaseThreshold, &keep);
+            cudaMemPoolSetAttribute(ctx->pool, cudaMemPoolAttrReleaseThreshold, &keep);
+            P.users.push_back(ctx);
         }
-        if (!ctx->uses_pool) ++P.users;
-        ctx->uses_pool = true;
     }
     b.bytes = bytes ? bytes : 16;
-    // the pool lives as long as a context that uses it
-    const int st = cuda_check(ctx, cudaMallocFromPoolAsync(&b.p, b.bytes, P.pool, s), "cudaMallocFromPoolAsync");
+    const int st = cuda_check(ctx, cudaMallocFromPoolAsync(&b.p, b.bytes, ctx->pool, s), "cudaMallocFromPoolAsync");
     if (st) b = DevBuf{};
     return st;
 }
@@ -122,7 +119,19 @@ int pool_upload(bsg_ctx *ctx, DevBuf &b, const void *src, size_t bytes, cudaStre
     return cuda_check(ctx, cudaMemcpyAsync(b.p, src, bytes, cudaMemcpyHostToDevice, s), "upload");
 }
 
-void pool_free(std::initializer_list<DevBuf *> bufs, cudaStream_t s) {
+// gives back what c's pool keeps (DevicePools::mu held); frees count as done once
+// the host has seen their stream end
+static void trim_one(bsg_ctx *c) {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (!c->pool_kept || cudaStreamIsCapturing(c->pool_stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone)
+        return;   // nothing, or a batch's stream that is capturing its iteration
+    if (cudaStreamSynchronize(c->pool_stream) != cudaSuccess || cudaMemPoolTrimTo(c->pool, 0) != cudaSuccess)
+        cudaGetLastError();
+    c->pool_kept = 0;
+    c->pool_most = 0;
+}
+
+void pool_free(bsg_ctx *ctx, std::initializer_list<DevBuf *> bufs, cudaStream_t s) {
     size_t bytes = 0;
     for (DevBuf *b : bufs) {
         if (b->p) {
@@ -131,30 +140,42 @@ void pool_free(std::initializer_list<DevBuf *> bufs, cudaStream_t s) {
         }
         *b = DevBuf{};
     }
+    if (!ctx->pool) return;
     // what lies above the pool's threshold goes back to the device at the
     // stream's next synchronization: here, not at some later call
     if (bytes > kPoolKeep) cudaStreamSynchronize(s);
+    DevicePools &P = g_pools[ctx->device];
+    std::lock_guard<std::mutex> lock(P.mu);
+    ctx->pool_stream = s;
+    if (P.users.back() != ctx) {
+        P.users.erase(std::find(P.users.begin(), P.users.end(), ctx));
+        P.users.push_back(ctx);
+    }
+    if (bytes <= ctx->pool_most) return;   // the pool has not grown
+    ctx->pool_most = bytes;
+    cudaMemPoolGetAttribute(ctx->pool, cudaMemPoolAttrReservedMemCurrent, &ctx->pool_kept);
+    uint64_t sum = 0;
+    for (const bsg_ctx *c : P.users) sum += c->pool_kept;
+    for (size_t k = 0; k + 1 < P.users.size() && sum > kPoolKeep; ++k) {
+        sum -= P.users[k]->pool_kept;
+        trim_one(P.users[k]);
+    }
 }
 
 void pool_trim(int device) {
     if (device < 0 || device >= kMaxDevices) return;
-    DevicePool &P = g_pools[device];
+    DevicePools &P = g_pools[device];
     std::lock_guard<std::mutex> lock(P.mu);
-    if (!P.pool) return;
-    // frees count as done once the host has seen their streams end
-    if (cudaDeviceSynchronize() != cudaSuccess || cudaMemPoolTrimTo(P.pool, 0) != cudaSuccess) cudaGetLastError();
+    for (bsg_ctx *c : P.users) trim_one(c);
 }
 
-// a context leaves its device's pool; the last one takes it down
 static void pool_leave(bsg_ctx *ctx) {
-    if (!ctx->uses_pool) return;
-    ctx->uses_pool = false;
-    DevicePool &P = g_pools[ctx->device];
+    if (!ctx->pool) return;
+    DevicePools &P = g_pools[ctx->device];
     std::lock_guard<std::mutex> lock(P.mu);
-    if (--P.users == 0) {
-        cudaMemPoolDestroy(P.pool);
-        P.pool = nullptr;
-    }
+    P.users.erase(std::find(P.users.begin(), P.users.end(), ctx));
+    cudaMemPoolDestroy(ctx->pool);
+    ctx->pool = nullptr;
 }
 
 void build_tile_list(const bsg_ctx *ctx, int tp, std::vector<Tile> &tiles) {

@@ -224,7 +224,11 @@ struct bsg_ctx {
     std::map<int, bsg::ChunkTiles> chunk_tiles;
     cudaStream_t copy_stream = nullptr;
     std::vector<cudaEvent_t> chunk_ev;
-    bool uses_pool = false;   // counted among the users of its device's scratch pool
+    // scratch (pool_alloc): the stream and the most bytes of a call since it was
+    // last trimmed, and what it kept after that one
+    cudaMemPool_t pool = nullptr;
+    cudaStream_t pool_stream = nullptr;
+    uint64_t pool_most = 0, pool_kept = 0;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
 };
 
@@ -235,13 +239,16 @@ int dev_alloc(bsg_ctx *ctx, DevBuf &b, size_t bytes);
 void dev_free(DevBuf &b);
 int upload(bsg_ctx *ctx, DevBuf &b, const void *src, size_t bytes);
 // stream-ordered scratch of the state calls (adjoint, densities), freed on the
-// same stream: one pool per device, which keeps up to kPoolKeep between calls, for
-// all contexts together, and goes with the last context that used it
+// same stream.  Each context has a pool (one for all costs a call that follows
+// another context's a wait across streams: gradients of four states of sd 2p6n 363
+// -> 404 us); the pools of a device keep up to kPoolKeep in all, the ones used
+// longest ago giving theirs back first
 constexpr uint64_t kPoolKeep = (uint64_t)1 << 30;
 int pool_alloc(bsg_ctx *ctx, DevBuf &b, size_t bytes, cudaStream_t s);
 int pool_upload(bsg_ctx *ctx, DevBuf &b, const void *src, size_t bytes, cudaStream_t s);
-void pool_free(std::initializer_list<DevBuf *> bufs, cudaStream_t s);
-// gives back what the pool keeps (waits for the device)
+// at the end of a call
+void pool_free(bsg_ctx *ctx, std::initializer_list<DevBuf *> bufs, cudaStream_t s);
+// gives back what the pools of a device keep
 void pool_trim(int device);
 const TileSet *get_tiles(bsg_ctx *ctx, int tp);
 // row tiles of width tp in longest-processing-time order (host list)

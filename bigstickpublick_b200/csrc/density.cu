@@ -470,7 +470,7 @@ static int density1b(bsg_ctx *ctx, const bsg_density_tables *dt, const double *v
     DevBuf d_cols, d_x, d_segs, d_chunks, d_part, d_l0, d_lid, d_outp, d_outn;
     cudaStream_t s = ctx->stream;
     auto release = [&]() {
-        pool_free({&d_cols, &d_x, &d_segs, &d_chunks, &d_part, &d_l0, &d_lid, &d_outp, &d_outn}, s);
+        pool_free(ctx, {&d_cols, &d_x, &d_segs, &d_chunks, &d_part, &d_l0, &d_lid, &d_outp, &d_outn}, s);
     };
     const size_t vbytes = sizeof(double) * (size_t)dim * ns;
     const bool direct = rows && ns == den_nsp(ns);   // already as staged

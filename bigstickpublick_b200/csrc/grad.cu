@@ -200,7 +200,7 @@ int grad_many(bsg_ctx *const *ctxs, int nsys, const double *const *evecs, int ns
     }
     bsg_ctx *c0 = ctxs[0];
     DevBuf psi, tmp, acc, out, descb, itemb, nnb, nnrb;
-    auto cleanup = [&]() { pool_free({&psi, &tmp, &acc, &out, &descb, &itemb, &nnb, &nnrb}, s); };
+    auto cleanup = [&]() { pool_free(c0, {&psi, &tmp, &acc, &out, &descb, &itemb, &nnb, &nnrb}, s); };
     int st;
     if (nstates == 1) rows = false;   // the same layout
     // row-major states come in so many basis states at a time, so that they do

@@ -273,9 +273,9 @@ int  bsg_grad(bsg_ctx *ctx, const double *evecs, int nstates,
 int  bsg_grad_rows(bsg_ctx *ctx, const double *evecs, int nstates,
               double *dpp, double *dnn, double *dpn, double *dspe_p, double *dspe_n);
 /*      Device scratch of this call and of bsg_density1b comes from a pool of the
- *      device, which keeps at most 1 GiB between calls for all contexts together
- *      and gives it back when the last context that used it is destroyed, or when
- *      another allocation of this library needs it. */
+ *      context.  The pools of a device keep at most 1 GiB in all between calls;
+ *      a context's goes with it, and all are given back when another allocation
+ *      of this library needs the memory. */
 /*      All states in one call.  The products of a label are added in FP64 inside
  *      a fixed group (a warp's positions, 16 rows of an NN operator) and the
  *      groups exactly (to 2^-64) in 128-bit fixed point with integer atomics, so
