@@ -15,11 +15,11 @@
 #include <atomic>
 #include <cstdio>
 #include <cstring>
+#include <mutex>
 #include <new>
 #include <numeric>
 #include <set>
 #include <thread>
-#include <mutex>
 #include <unordered_map>
 
 #include "bsg_internal.h"
@@ -123,8 +123,11 @@ int pool_upload(bsg_ctx *ctx, DevBuf &b, const void *src, size_t bytes, cudaStre
 // the host has seen their stream end
 static void trim_one(bsg_ctx *c) {
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    if (!c->pool_kept || cudaStreamIsCapturing(c->pool_stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone)
-        return;   // nothing, or a batch's stream that is capturing its iteration
+    if (!c->pool_kept) return;
+    if (cudaStreamIsCapturing(c->pool_stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
+        cudaGetLastError();
+        return;   // a batch's stream that is capturing its iteration
+    }
     if (cudaStreamSynchronize(c->pool_stream) != cudaSuccess || cudaMemPoolTrimTo(c->pool, 0) != cudaSuccess)
         cudaGetLastError();
     c->pool_kept = 0;

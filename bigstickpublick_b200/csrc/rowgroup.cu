@@ -157,8 +157,8 @@ GroupShape group_shape(const bsg_ctx *ctx, int esize, int nv) {
 //    1.03) and, where the rows fill the chip twice, at four (pf 4p3n ... 6p3n: FP64
 //    nb = 8 0.95 - 0.97, FP32 nb = 16 0.97 - 0.99; pf 3p3n, 1,140 rows, 1.02; sd
 //    1.01 - 1.14); the groups elsewhere (FP32 nb = 4 1.05 - 1.5, FP64 nb = 16 1.09 -
-//    2).  Spaces of some dozen rows scatter: sd 2p6n loses at FP32 nb = 16 (0.78)
-//    what sd 2p8n gains (1.26).
+//    2).  Spaces of few rows scatter: sd 2p6n (66 rows) loses at FP32 nb = 16 (0.78)
+//    what sd 2p8n gains (1.26), sd 3p6n (220) at nb = 4 (0.94) what sd 3p7n (1.21).
 bool group_takes(const bsg_ctx *ctx, int nb, int prec) {
     if (!ctx->grouped) return false;
     if (nb == 1 || group_shape(ctx, prec, 1).parts == 1) return true;
