@@ -13,6 +13,7 @@
 
 #include <algorithm>
 #include <atomic>
+#include <cmath>
 #include <cstdio>
 #include <cstring>
 #include <mutex>
@@ -1069,13 +1070,12 @@ int derive(bsg_ctx *ctx, const bsg_tables *t, const bsg_tables3 *t3, bool do_upl
                 slice_off_all[op.slice_base + sl] = (int32_t)off;
                 const size_t row0 = (size_t)(op.sell_base + off);
                 // unused places: the jump-group kernel reads them as a record
-                // of a position (one past the operator's input positions, one
-                // past the longest row) and, in a PN operator, of a label (one
-                // past its own) that it keeps zero; the row-tile kernels count
-                // records and never read them (nor are they read where the
-                // fields are too narrow: group_eligible)
+                // of a position that it keeps zero (one past the operator's
+                // input positions, one past the longest row); the row-tile
+                // kernels count records and never read them (nor are they read
+                // where 16 bits are too few: group_eligible)
                 const int32_t zero_pos = op.kind == 1 ? nop_maxin[o] + 1 : ctx->max_rowlen;
-                const uint32_t zero32 = ((uint32_t)zero_pos & 0xffffu) | ((uint32_t)(op.kind == 1 ? op.nbd : 0) & 0x7fffu) << 16;
+                const uint32_t zero32 = (uint32_t)zero_pos & 0xffffu;
                 for (size_t q = row0; q < row0 + (size_t)32 * width; ++q) {
                     sell_all[q] = make_int2(zero_pos, 0);
                     if (pack32) sell32_all[q] = zero32;
@@ -1342,7 +1342,8 @@ int derive(bsg_ctx *ctx, const bsg_tables *t, const bsg_tables3 *t3, bool do_upl
     a.nspe = (const float *)ctx->nspe.p;
     a.ld_cpn = ld;
     a.ncpn = (int32_t)cpn32.size();
-    const GroupSource gs{nops, nop_maxin, nptr_all, spe_ptr, pn};
+    const bool finite = std::all_of(hpn.begin(), hpn.end(), [](float x) { return std::isfinite(x); });
+    const GroupSource gs{nops, nop_maxin, nptr_all, spe_ptr, pn, finite};
     if (!group_eligible(ctx, gs, pack32)) return BSG_OK;
     // the groups come on top of the row tiles' tables, which are complete:
     // where they do not fit in memory or in their indexes, the row tiles take

@@ -128,7 +128,7 @@ GroupShape group_shape(const bsg_ctx *ctx, int esize, int nv) {
     GroupShape r;
     const int64_t j = esize == 4 && nv == 1 ? 4 : 2;
     r.accel = ((ctx->max_rowlen + 31) & ~31) * nv;
-    r.bufel = (int)((std::max<int64_t>(j * (ctx->group_nbd + 1) + j * nv * (ctx->group_nin + 1), (int64_t)nv * (ctx->max_rowlen + 1)) + 3) &
+    r.bufel = (int)((std::max<int64_t>(j * ctx->group_nbd + j * nv * (ctx->group_nin + 1), (int64_t)nv * (ctx->max_rowlen + 1)) + 3) &
                     ~(int64_t)3);
     const size_t b = r.part_bytes(esize);
     const size_t one = nv == 1 ? b : group_shape(ctx, esize, 1).part_bytes(esize);
@@ -183,9 +183,13 @@ bool group_eligible(bsg_ctx *ctx, const GroupSource &S, bool pack32) {
             ctx->group_nbd = std::max<int64_t>(ctx->group_nbd, S.nops[o].nbd);
             ctx->group_nin = std::max<int64_t>(ctx->group_nin, S.nop_maxin[o] + 1);
         }
-    // a record has 16 bits for the position and 15 for the label, one of each past
-    // the operator's own for the unused places
-    if (ctx->max_rowlen > 65535 || ctx->group_nbd > 32767) return false;
+    // unused record places read a zero input and the operator's first element: an
+    // infinite one would reach positions that it does not couple.  (A zero element
+    // of their own, staged for each group, costs 3 % on three-body pf 2p3n FP64.)
+    if (!S.finite) return false;
+    // a record has 16 bits for the position, one past the operator's own inputs for
+    // the unused places
+    if (ctx->max_rowlen > 65535) return false;
     // few long rows (one CTA of a few warps each) do not fill the chip, where
     // the row-tile kernel cuts them (pf 2p4n, 190 rows: FP64 159 us against 88)
     for (int esize : {4, 8}) {

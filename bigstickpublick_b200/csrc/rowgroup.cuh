@@ -117,10 +117,7 @@ __device__ __forceinline__ void group_walk(const RowArgs &a, const GroupArgs &g,
             X[i * xs + n] = x;
         }
     }
-    // what the unused record places read: an input and an element of their own, both
-    // zero (a label of the operator may hold an infinite element)
-    if (tid < NA) X[tid * xs + nin] = XJ{};
-    if (tid == 0) V[op.nbd] = VJ{};
+    if (tid < NA) X[tid * xs + nin] = XJ{};   // what the unused record places read
     pt.sync();
     const int32_t *__restrict__ so = a.slice_off + op.slice_base;
     const uint32_t *__restrict__ recs = a.sell32 + op.sell_base + pt.lane;

@@ -19,6 +19,7 @@ struct GroupSource {
     const std::vector<int32_t> &nptr;
     const std::vector<int32_t> &spe_ptr;
     const std::vector<std::pair<int32_t, PNContrib>> &pn;
+    bool finite;   // every element of hmatpn (hmatppn, hmatpnn) is
 };
 // whether the context takes the jump-group kernel
 bool group_eligible(bsg_ctx *ctx, const GroupSource &S, bool pack32);
