@@ -1,9 +1,9 @@
 """A matrix element that is not finite reaches the outputs that it couples and no
-others: the unused record places of the jump groups, which read an element beside a
-zero input, are not met by such contexts.  Twelve labels are tried one by one, each the one that a PN bundle's
-first proton and first neutron jump use (the first element of the jump's row of
-elements); the outputs' finite, infinite and not-a-number places must be the
-oracle's."""
+others: contexts with one stay on the row tiles, which do not read the unused record
+places that the jump groups multiply with a zero input.  Twelve labels are tried one
+by one, each the one that a PN bundle's first proton and first neutron jump use (the
+first element of the jump's row of elements); the outputs' finite, infinite and
+not-a-number places must be the oracle's."""
 import numpy as np
 import pytest
 
